@@ -418,30 +418,19 @@ int sgb_sim_profile(sgb_sim* sim, int32_t n_steps, double* mean_us, double* byte
  * outside it); a simulation that needs every spike to land in its own future
  * slot keeps all delays < ring_slots.  All pointers are device pointers; work is enqueued on `stream` (a
  * cudaStream_t as void*, NULL = legacy default stream) and the call returns
- * without waiting.  Scratch for the active-cell list is taken from the
- * stream-ordered pool (cudaMallocAsync) and released on the same stream. */
+ * without waiting.  One kernel, no scratch memory: calls on different streams
+ * or threads only share what the caller makes them share. */
 int sgb_deliver_spikes(const uint8_t* spikes, int32_t n_cells, const uint32_t* row,
                        const uint32_t* syn, const void* weights, int32_t weight_type,
                        int32_t* ring, int32_t ring_slots, int64_t step, void* stream);
 
-/* Same operation as sgb_deliver_spikes, allocating nothing.  This entry point
- * has no counterpart in the reference.  It is for callers that cannot
- * allocate device memory when they deliver spikes: a real-time step loop in
- * which a device allocation (which may synchronise the device) would break
- * the deadline, or a process whose device memory belongs to another allocator
- * (a framework's caching allocator, a fixed budget) that must not be bypassed.
- * The caller passes inputs and outputs as above; the scratch (one count word
- * and the list of active cells) is a file-scope device array of the library,
- * sized for n_cells <= 1,048,576 (4 MiB), which every GPU that loads the
- * library holds until the process exits.  Larger n_cells return
- * SGB_ERR_RANGE.  The first call on a device looks up that array's device
- * address (cudaGetSymbolAddress) with the device current; make that first
- * call before any stream capture.  A cudaDeviceReset of that device ends the
- * context holding the array, so the cached address is stale afterwards: do
- * not call this entry point on a device the process has reset.  Every call
- * clears the count word on its stream and shares the one array, so calls
- * that overlap on the GPU (other streams, other host threads) race:
- * serialise them. */
+/* Same operation as sgb_deliver_spikes for callers that cannot allocate device
+ * memory when they deliver spikes: a real-time step loop in which a device
+ * allocation (which may synchronise the device) would break the deadline, or
+ * a process whose device memory belongs to another allocator (a framework's
+ * caching allocator, a fixed budget) that must not be bypassed.  This entry
+ * point has no counterpart in the reference.  Neither entry point allocates;
+ * this one takes n_cells <= 1,048,576 and returns SGB_ERR_RANGE beyond. */
 int sgb_deliver_spikes_static(const uint8_t* spikes, int32_t n_cells, const uint32_t* row,
                               const uint32_t* syn, const void* weights, int32_t weight_type,
                               int32_t* ring, int32_t ring_slots, int64_t step, void* stream);
