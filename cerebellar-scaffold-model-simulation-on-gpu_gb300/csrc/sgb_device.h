@@ -178,6 +178,8 @@ struct StepArgs {
   unsigned long long* recent;     // [2][n_pad] per-cell spike registers (plasticity), or NULL:
                                   // the update of step t writes buffer t & 1 (bit j = step
                                   // t - j) from buffer (t - 1) & 1
+  unsigned long long* recent3;    // [3][n_pad] the same, step mod 3, inside a k_persistent_pull
+                                  // launch; NULL unless every plastic window fits the registers
   uint32_t* hsum;                 // [H + 1][n_swords]: bit w of row t mod (H + 1) = word w
                                   // of step t had a spike
   uint2* items;                   // [2][item_cap] push work ranges
@@ -206,6 +208,8 @@ struct StepArgs {
   uint32_t any_push;
   uint32_t raster_cap;
   uint32_t item_cap;              // items per parity buffer
+  uint32_t pull_smem;             // k_persistent_pull: dynamic shared memory (0: not run)
+  uint32_t pull_held;             // its pull units per block with entries in shared memory
   uint32_t row_smem;              // fused persistent kernel: shared-memory bytes for push rows (0: none)
   uint32_t n_shards;              // fused persistent kernel: deferred shards (0: none)
   uint32_t shard_grid;            // the grid size the shards were dealt for
@@ -229,6 +233,9 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
 uint32_t fused_row_smem_max();
 cudaError_t set_fused_row_smem(uint32_t bytes);
 int persistent_blocks_per_sm(bool bf16);
+// Whether resident networks with dense pulls run k_persistent_pull, and its
+// shared memory (a.pull_smem, a.pull_held), for the handle's current modes.
+void plan_persistent_pull(StepArgs& a, int blocks);
 // Dense pull (per-step driver): k_pull needs pull_setup() once per device
 // before its first launch.
 cudaError_t launch_pull(const StepArgs& a, int blocks, cudaStream_t s);

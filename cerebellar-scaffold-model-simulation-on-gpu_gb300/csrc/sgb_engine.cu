@@ -256,6 +256,7 @@ static int upload_modes(Sim& s) {
     SGB_CUDA(cudaMemcpy((void*)a.pull_units, units.data(), units.size() * sizeof(PullUnit), cudaMemcpyHostToDevice));
   SGB_CUDA(cudaMemcpy((void*)a.projs, s.projs.data(), s.projs.size() * sizeof(ProjDev), cudaMemcpyHostToDevice));
   a.n_pull_units = (uint32_t)units.size();
+  plan_persistent_pull(a, s.persistent_blocks);
   // Fused persistent kernel.  Shards: the delay >= 3 parts of long rows
   // (longest first) are cut into kPushChunk-synapse shards dealt round-robin
   // over the blocks, so one spike's pushes spread over many SMs; a cell whose
@@ -698,6 +699,8 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
     bytes = align_up(bytes + std::max<size_t>(units.size(), 1) * sizeof(PullUnit), 256);
     s.off_recent = bytes;
     bytes = align_up(bytes + (size_t)s.n_pad * 16, 256);  // two buffers
+    const size_t off_recent3 = bytes;
+    if (may_fuse) bytes = align_up(bytes + (size_t)s.n_pad * 24, 256);
     std::vector<size_t> off_w0(s.plast.size()), off_t(s.plast.size());
     for (size_t i = 0; i < s.plast.size(); ++i) {
       PlastHost& ph = s.plast[i];
@@ -761,6 +764,9 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
       SGB_CUDA(cudaMemcpy(pb + off_units, units.data(), units.size() * sizeof(PullUnit), cudaMemcpyHostToDevice));
     a.plast = (const PlastDev*)pb;
     a.recent = (unsigned long long*)(pb + s.off_recent);
+    bool windows_ok = may_fuse;  // resident, and every window from the spike registers
+    for (const PlastDev& d : pd) windows_ok = windows_ok && d.recent_ok;
+    a.recent3 = windows_ok ? (unsigned long long*)(pb + off_recent3) : nullptr;
     a.n_plast = (uint32_t)pd.size();
     a.stdp_early = 1u;  // the Teacher rule reads its teacher's and pre cells' earlier spikes
     for (const PlastDev& d : pd)

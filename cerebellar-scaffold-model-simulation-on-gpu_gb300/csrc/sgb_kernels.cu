@@ -1014,23 +1014,30 @@ __device__ __forceinline__ uint32_t hist_bit(const uint32_t* hb, uint32_t off) {
 // (four per lane, loads issued together), so the rows of the few posts that
 // do change spread over many warps; the window's spike count is gathered
 // eight rows at a time.
-template <bool BF16, bool COH>
-__device__ __forceinline__ bool stdp_post_spiked(const StepArgs& a, const PlastDev& L,
-                                                 const ProjDev& P, const uint32_t* hb,
+// Hist: where a spike bit at an offset above the step's history row is read
+// (HistGlobal, or the rows a block keeps in shared memory).
+template <bool COH>
+struct HistGlobal {
+  const uint32_t* hb;
+  __device__ __forceinline__ uint32_t bit(uint32_t off) const { return hist_bit<COH>(hb, off); }
+};
+
+template <class Hist>
+__device__ __forceinline__ bool stdp_post_spiked(const PlastDev& L, const ProjDev& P, const Hist& h,
                                                  uint32_t post) {
   const uint32_t so = L.rule == SGB_STDP_TEACHER ? __ldg(L.teacher + post) : P.post_base + post;
-  return so != 0xFFFFFFFFu && hist_bit<COH>(hb, so);
+  return so != 0xFFFFFFFFu && h.bit(so);
 }
 
 // Updates the cells of one unit (the whole warp, four cells per lane).
 // EARLY: run during the update of step t (a rule that reads only earlier
-// steps' spikes), so the spike registers are read from the buffer of step
-// t - 1, one bit lower.
+// steps' spikes), so `recent`, the spike registers, are those of step t - 1,
+// read one bit lower; else those of step t.
 // spiked: the screening found the unit inside one post cell's row with its
 // post / teacher spike set, so the entries need not look it up again.
-template <bool BF16, bool COH, bool EARLY>
-__device__ __forceinline__ void stdp_unit(const StepArgs& a, const PullUnit un,
-                                          const uint32_t* hb, uint32_t pad, unsigned long long t,
+template <bool BF16, bool COH, bool EARLY, class Hist>
+__device__ __forceinline__ void stdp_unit(const StepArgs& a, const PullUnit un, const Hist& h,
+                                          uint32_t pad, const unsigned long long* recent,
                                           bool spiked = false) {
   constexpr uint32_t B = kStdpUnit / 32;
   const uint32_t lane = threadIdx.x & 31u;
@@ -1049,8 +1056,7 @@ __device__ __forceinline__ void stdp_unit(const StepArgs& a, const PullUnit un,
   for (uint32_t k = 0; k < B; ++k) {
     const uint32_t o = un.o0 + lane + 32u * k;
     sp[k] = e[k] < pad &&
-            (spiked ||
-             stdp_post_spiked<BF16, COH>(a, L, P, hb, P.ell_rowmajor ? o / P.ell_K : o % P.post_count));
+            (spiked || stdp_post_spiked(L, P, h, P.ell_rowmajor ? o / P.ell_K : o % P.post_count));
   }
 #pragma unroll
   for (uint32_t k = 0; k < B; ++k) {
@@ -1063,19 +1069,19 @@ __device__ __forceinline__ void stdp_unit(const StepArgs& a, const PullUnit un,
       // The pre cell's spike register: bit d is step t - d, bits d .. d +
       // window - 1 the window (d + window <= 64 for this projection).
       const uint32_t d = e[k] / a.n_pad + 1u, g = e[k] - (d - 1u) * a.n_pad;
-      const unsigned long long* rb = a.recent + ((EARLY ? t + 1ull : t) & 1ull) * a.n_pad + g;
+      const unsigned long long* rb = recent + g;
       const unsigned long long r = (COH ? __ldcg(rb) : __ldg(rb)) >> (EARLY ? d - 1u : d);
       s_pre = (r & 1ull) != 0ull;
       if (sp[k] && L.a2_ji != 0.f)
         nwin = __popcll(L.window == 64u ? r : r & ((1ull << L.window) - 1ull));
     } else {
-      s_pre = hist_bit<COH>(hb, e[k] + a.n_pad) != 0u;
+      s_pre = h.bit(e[k] + a.n_pad) != 0u;
       if (sp[k] && L.a2_ji != 0.f) {
         for (uint32_t j0 = 0; j0 < L.window; j0 += 8u) {
           uint32_t bit[8];
 #pragma unroll
           for (uint32_t j = 0; j < 8u; ++j)
-            bit[j] = j0 + j < L.window ? hist_bit<COH>(hb, e[k] + (j0 + j + 1u) * a.n_pad) : 0u;
+            bit[j] = j0 + j < L.window ? h.bit(e[k] + (j0 + j + 1u) * a.n_pad) : 0u;
 #pragma unroll
           for (uint32_t j = 0; j < 8u; ++j) nwin += bit[j];
         }
@@ -1112,8 +1118,9 @@ template <bool BF16, bool COH, bool EARLY>
 __device__ __forceinline__ void stdp_warp(const StepArgs& a, uint32_t gw, uint32_t nw,
                                           const StepIdx& ix) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t* hb = hist_base(a, ix.hrow);
+  const HistGlobal<COH> hb{hist_base(a, ix.hrow)};
   const uint32_t pad = a.hist_rows * a.n_pad;
+  const unsigned long long* recent = a.recent + ((EARLY ? ix.t + 1ull : ix.t) & 1ull) * a.n_pad;
   for (uint32_t base = gw; base < a.n_stdp_units; base += 32u * nw) {
     const uint32_t u = base + lane * nw;
     bool active = false, one = false;  // one: a single post, whose post / teacher spike is set
@@ -1126,7 +1133,7 @@ __device__ __forceinline__ void stdp_warp(const StepArgs& a, uint32_t gw, uint32
       } else {
         const uint32_t end = min(un.o0 + kStdpUnit, P.ell_n);
         const uint32_t p0 = un.o0 / P.ell_K, p1 = (end - 1u) / P.ell_K;
-        for (uint32_t p = p0; p <= p1; ++p) active |= stdp_post_spiked<BF16, COH>(a, L, P, hb, p);
+        for (uint32_t p = p0; p <= p1; ++p) active |= stdp_post_spiked(L, P, hb, p);
         one = active && p0 == p1;
       }
     }
@@ -1135,7 +1142,7 @@ __device__ __forceinline__ void stdp_warp(const StepArgs& a, uint32_t gw, uint32
     while (act) {
       const uint32_t j = __ffs(act) - 1;
       act &= act - 1;
-      stdp_unit<BF16, COH, EARLY>(a, a.stdp_units[base + j * nw], hb, pad, ix.t, (ones >> j) & 1u);
+      stdp_unit<BF16, COH, EARLY>(a, a.stdp_units[base + j * nw], hb, pad, recent, (ones >> j) & 1u);
     }
   }
 }
@@ -1269,6 +1276,12 @@ __device__ __forceinline__ bool grid_barrier(const StepArgs& a, unsigned long lo
 
 __host__ __device__ __forceinline__ size_t seg_smem_bytes_dev(const StepArgs& a) {
   return seg_table_bytes(a.n_segs) + (((size_t)a.n_srcs * sizeof(SrcDev) + 15) & ~(size_t)15);
+}
+
+// History rows k_persistent_pull keeps: the delay rows of a pull, and one more
+// for a teacher max_delay steps back.
+__host__ __device__ __forceinline__ uint32_t pull_rows(const StepArgs& a) {
+  return a.max_delay + (a.n_plast ? 1u : 0u);
 }
 
 // Raster offsets of a launch with one grid barrier per step: a block may
@@ -1507,6 +1520,287 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_resident(StepAr
   if (valid && lif) state_out(a, i, st);
   if (__ldcg(&ctl->error) & kErrBarrierTimeout) return;
   if (lane == 0 && walked) atomicAdd(&ctl->delivered, (unsigned long long)walked);
+  if (leader) {
+    ctl->step = t0 + n_steps;
+    ctl->ring_slot = ix.slot;
+    ctl->hist_row = ix.hrow;
+    ctl->t_rel = n_steps;
+  }
+}
+
+// Resident form with dense pulls, one substep a step: one grid barrier a step.
+// The reference tests a spike on the potential before the step's integration,
+// so the spikes of step t + 1 are known when step t's update ends.  Iteration t
+// publishes them (as the fused kernel's late-push timelines do) and, in the
+// same phase, pulls into slot t + 1 from the spikes of steps <= t, which the
+// previous barrier completed: nothing in an iteration waits for another
+// block's work of the same iteration.
+//   The pull reads no table from global memory: a block keeps the entries of
+// its units (unit u belongs to block u mod blocks) in shared memory for the
+// whole launch, as many as fit, beside the D history rows a pull reads; an
+// iteration loads only the row of step t (n_words words) and tests every entry
+// on its own bit, so only deliveries leave the SM: their weight and one
+// reduction.  The rows also free the writers of row t + 1 from readers of
+// row t + 1 - H.
+//   Plastic projections: the block that pulls a unit also updates its weights,
+// so a block barrier orders the two.  Rules that read only earlier steps'
+// spikes (stdp_early) make the update of step t + 1 behind iteration t's
+// barrier arrival, the others that of step t before its pulls.  The spike
+// registers stay in their owners' registers and are published in three
+// buffers (step mod 3): behind the arrival, faster blocks already write those
+// of step t + 2 while step t's are read.
+//   What bounds it is latency: ring slot and history row (one L2 round trip),
+// the test of 18 entries a thread, weight, reduction, barrier.  92,550 cells,
+// every projection dense, 16-bit weights: 9.0 us per step with two barriers and
+// the entries read from L2 -> 4.6 us; Teacher rule on 1.75M synapses 10.2 ->
+// 6.1 us.
+struct HistRows {     // rows of the last steps, newest at word `base`, in decreasing step order
+  const uint32_t* s;
+  uint32_t base, total;  // total: words of all rows (the rows are a ring)
+  __device__ __forceinline__ uint32_t word(uint32_t w) const {
+    const uint32_t x = base + w;
+    return s[min(x, x - total)];
+  }
+  __device__ __forceinline__ uint32_t bit(uint32_t off) const {
+    return (word(off >> 5) >> (off & 31u)) & 1u;
+  }
+};
+
+// The plasticity of a step on the block's own units (h and recent as the step
+// sees them): threads screen sub-units of kStdpUnit cells, then warps update the ones that can change.  The caller's
+// block barriers order it against the block's pulls; *s_n is 0 on entry.
+template <bool BF16, bool EARLY>
+__device__ __forceinline__ void stdp_own(const StepArgs& a, const HistRows& h,
+                                         const unsigned long long* recent, uint32_t* s_list,
+                                         uint32_t* s_n) {
+  constexpr uint32_t kSub = kPullUnit / kStdpUnit;
+  const uint32_t pad = a.hist_rows * a.n_pad;
+  const uint32_t mine = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x;
+  for (uint32_t b = 0; b < mine * kSub; b += kPersistBlock) {
+    const uint32_t x = b + threadIdx.x;
+    if (x < mine * kSub) {
+      const PullUnit pu = a.pull_units[blockIdx.x + (x / kSub) * gridDim.x];
+      const uint32_t o0 = pu.o0 + (x % kSub) * kStdpUnit;
+      for (uint32_t k = 0; k < a.n_plast; ++k) {
+        const PlastDev& L = a.plast[k];
+        const ProjDev& P = a.projs[L.proj];
+        if (L.proj != pu.proj || o0 >= P.ell_n) continue;
+        bool active = L.a0 != 0.f || L.a1_j != 0.f || !P.ell_rowmajor, one = false;
+        if (!active) {
+          const uint32_t p0 = o0 / P.ell_K, p1 = (min(o0 + kStdpUnit, P.ell_n) - 1u) / P.ell_K;
+          for (uint32_t p = p0; p <= p1; ++p) active |= stdp_post_spiked(L, P, h, p);
+          one = active && p0 == p1;
+        }
+        if (active) s_list[atomicAdd(s_n, 1u)] = threadIdx.x | (k << 16) | (one ? 1u << 31 : 0u);
+      }
+    }
+    __syncthreads();
+    const uint32_t n = *s_n;
+    for (uint32_t j = threadIdx.x >> 5; j < n; j += kPersistBlock / 32) {
+      const uint32_t v = s_list[j], y = b + (v & 0xFFFFu);
+      const uint32_t o0 = a.pull_units[blockIdx.x + (y / kSub) * gridDim.x].o0;
+      stdp_unit<BF16, true, EARLY>(a, PullUnit{(v >> 16) & 0x7FFFu, o0 + (y % kSub) * kStdpUnit}, h, pad,
+                                   recent, v >> 31);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *s_n = 0;
+    __syncthreads();
+  }
+}
+
+template <bool BF16>
+__global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a, uint32_t n_steps) {
+  // Dynamic shared memory: segment descriptors and sources, the history rows,
+  // then the entries of the block's first a.pull_held units.
+  __shared__ uint2 s_items[kGenItems];
+  __shared__ uint32_t s_icnt[2];
+  __shared__ uint32_t s_wsum[kPersistBlock / 32];
+  __shared__ uint32_t s_act[kPersistBlock];  // active plastic sub-units
+  __shared__ uint32_t s_nact;
+  const uint32_t n_rows = pull_rows(a), row_words = n_rows * a.n_words;
+  uint32_t* s_hist = reinterpret_cast<uint32_t*>(g_dyn + seg_smem_bytes_dev(a));
+  uint4* s_ent = reinterpret_cast<uint4*>(s_hist + row_words);
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(a.segs);
+    uint4* dst = reinterpret_cast<uint4*>(g_dyn);
+    for (uint32_t j = threadIdx.x; j < a.n_segs * (uint32_t)(sizeof(SegDev) / 16); j += kPersistBlock)
+      dst[j] = src[j];
+    const uint2* ss = reinterpret_cast<const uint2*>(a.srcs);
+    uint2* sd = reinterpret_cast<uint2*>(g_dyn + seg_table_bytes(a.n_segs));
+    for (uint32_t j = threadIdx.x; j < a.n_srcs * (uint32_t)(sizeof(SrcDev) / 8); j += kPersistBlock)
+      sd[j] = ss[j];
+  }
+  const SegDev* segs = reinterpret_cast<const SegDev*>(g_dyn);
+  const SrcDev* srcs = reinterpret_cast<const SrcDev*>(g_dyn + seg_table_bytes(a.n_segs));
+  Ctl* ctl = a.ctl;
+  StepIdx ix = step_of(a);
+  const unsigned long long t0 = ix.t;
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
+  constexpr uint32_t kWarps = kPersistBlock / 32;
+  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+  // The rows of steps t0 - 1, t0 - 2, ...; row 0 (step t0) follows in the loop.
+  for (uint32_t j = a.n_words / 4u + threadIdx.x; j < row_words / 4u; j += kPersistBlock)
+    reinterpret_cast<uint4*>(s_hist)[j] = __ldcg(reinterpret_cast<const uint4*>(hist_base(a, ix.hrow)) + j);
+  // Entries; padding becomes pad1, which the ring of rows maps to row 0.
+  const uint32_t pad = a.hist_rows * a.n_pad, pad1 = n_rows * a.n_pad;
+  const uint32_t mine = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x;
+  const uint32_t held = min(mine, a.pull_held);
+  constexpr uint32_t kQ = kPullUnit / 4;  // 16-byte groups per unit
+  auto entries = [&](uint32_t q) -> uint4 {  // group q of the block's units, padding as pad1
+    const PullUnit un = a.pull_units[blockIdx.x + (q / kQ) * gridDim.x];
+    uint4 e = __ldg(reinterpret_cast<const uint4*>(a.projs[un.proj].ell_syn + un.o0) + q % kQ);
+    e.x = min(e.x, pad1); e.y = min(e.y, pad1); e.z = min(e.z, pad1); e.w = min(e.w, pad1);
+    return e;
+  };
+  for (uint32_t q = threadIdx.x; q < held * kQ; q += kPersistBlock) s_ent[q] = entries(q);
+  // Words are dealt round-robin over the blocks (word slot = warp x blocks + block).
+  const uint32_t ws = wib * gridDim.x + blockIdx.x;
+  const bool has = ws < a.n_upd_words;
+  uint32_t w = 0, seg = 0, i = 0, local = 0, mask = 0, r0 = 0, r1 = 0, od = 0;
+  bool valid = false, lif = false;
+  float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (has) {
+    w = __ldg(a.upd_words + ws);
+    seg = __ldg(a.seg_of_word + w);
+    i = (w << 5) + lane;
+    const SegDev& sd = a.segs[seg];
+    local = i - sd.base;
+    valid = local < sd.count;
+    lif = sd.kind == kSegLif;
+    if (valid) {
+      if (lif) st = state_in(a.su[i], a.sg[i], sd.Vr); else mask = __ldg(a.src_mask + i);
+      od = __ldg(a.outdeg + i);
+      if (a.any_push) {
+        r0 = __ldg(a.push_row + i);
+        r1 = __ldg(a.push_row + i + 1);
+      }
+    }
+  }
+  if (threadIdx.x == 0) s_icnt[0] = s_icnt[1] = s_nact = 0;
+  __syncthreads();
+  const bool stim = mask != 0u, rd = lif && valid;
+  unsigned long long target = 0;
+  uint32_t walked = 0, hits = 0;
+  int2* ring2 = reinterpret_cast<int2*>(a.ring);
+  unsigned long long reg = 0;  // the cell's spike register, bit j = step t - j
+  if (a.recent && valid) reg = a.recent[((t0 + 1ull) & 1ull) * a.n_pad + i];
+  uint32_t tri = (uint32_t)(t0 % 3ull);  // buffer of the last published step
+  // Publishes the spikes of step px.t (chunk row px.rel): bitmap, counts,
+  // spike register, and push items of parity par.
+  auto publish = [&](bool fired, const StepIdx& px, uint32_t par) {
+    if (!has) return;
+    if (a.recent && valid) {
+      reg = (reg << 1) | (fired ? 1ull : 0ull);
+      a.recent3[(size_t)tri * a.n_pad + i] = reg;
+    }
+    walked += publish_word<BF16, true>(a, w, seg, i, fired, r0, r1, od, px,
+                                       BlockItems{s_items, &s_icnt[par]});
+  };
+  auto push = [&](const StepIdx& px, uint32_t par) {  // after a block barrier
+    const uint32_t n_items = min(s_icnt[par], kGenItems);
+    if (threadIdx.x == 0) s_icnt[par ^ 1u] = 0;
+    for (uint32_t u = wib; u < n_items; u += kWarps) walked += push_item<BF16>(a, s_items[u], px.slot);
+  };
+  // Deliveries of one lane's hits in group q: bit j of `hit` is entry j.
+  auto deliver = [&](uint32_t q, uint32_t hit, uint32_t slot1) {
+    const PullUnit un = a.pull_units[blockIdx.x + (q / kQ) * gridDim.x];
+    const ProjDev& P = a.projs[un.proj];
+    while (hit) {
+      const uint32_t j = __ffs(hit) - 1u;
+      hit &= hit - 1u;
+      ++hits;
+      pull_hit<BF16>(a, P, un.o0 + (q % kQ) * 4u + j, slot1);
+    }
+  };
+  auto test4 = [&](const HistRows& h, uint4 e) -> uint32_t {
+    const uint32_t v = h.bit(e.x) | (h.bit(e.y) << 1) | (h.bit(e.z) << 2) | (h.bit(e.w) << 3);
+    // A padding entry reads some bit of row 0; it is told apart only on a hit.
+    return v == 0u ? 0u
+                   : v & ((e.x < pad1 ? 1u : 0u) | (e.y < pad1 ? 2u : 0u) | (e.z < pad1 ? 4u : 0u) |
+                          (e.w < pad1 ? 8u : 0u));
+  };
+  const auto draw = [&](unsigned long long t) {
+    return stim && input_fire(a, srcs, segs[seg], local, mask, t);
+  };
+  HistRows rows{s_hist, 0u, row_words};  // newest row: step t
+  bool in_next = false, aborted = false;
+  if (n_steps) {
+    if (a.n_plast && a.stdp_early)
+      stdp_own<BF16, true>(a, rows, a.recent + ((t0 + 1ull) & 1ull) * a.n_pad, s_act, &s_nact);
+    ix.rel = 0;
+    clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
+    publish(valid && (lif ? st.x > segs[seg].Vth : draw(t0)), ix, 0u);
+    __syncthreads();
+    push(ix, 0u);
+    grid_arrive(a, target);
+    if (n_steps > 1) in_next = draw(t0 + 1ull);
+    aborted = !grid_wait(a, target);
+  }
+  for (uint32_t s = 0; s < n_steps && !aborted; ++s) {
+    const bool more = s + 1u < n_steps;
+    // Row of step t and ring slot t: one round trip for both.
+    const uint4* src = reinterpret_cast<const uint4*>(hist_base(a, ix.hrow));
+    uint4* dst = reinterpret_cast<uint4*>(s_hist + rows.base);
+    const uint32_t n4 = a.n_words / 4u;
+    uint4 hv = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < n4) hv = __ldcg(src + threadIdx.x);
+    int2 acc = make_int2(0, 0);
+    if (rd) acc = __ldcg(ring2 + (ix.roff + i));
+    const uint32_t consumed = ix.roff;
+    for (uint32_t j = kPersistBlock + threadIdx.x; j < n4; j += kPersistBlock) dst[j] = __ldcg(src + j);
+    if (threadIdx.x < n4) dst[threadIdx.x] = hv;
+    // From here on ix is step t + 1, whose spikes this step publishes.
+    ix.t += 1ull;
+    ix.rel = s + 1u;
+    ix_advance(a, ix);
+    clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
+    const unsigned long long* rec_t = a.recent3 + (size_t)tri * a.n_pad;  // registers of step t
+    if (more) tri = tri == 2u ? 0u : tri + 1u;
+    bool fired = in_next;
+    if (has && lif) {
+      const LifK k = lif_k(segs[seg]);
+      if (rd) lif_update<1>(k, 1, st, acc);
+      fired = valid && st.x > k.Vth;
+      if (acc.x | acc.y) __stcg(ring2 + (consumed + i), make_int2(0, 0));
+    }
+    const uint32_t par = (s + 1u) & 1u;
+    if (more) publish(fired, ix, par);
+    __syncthreads();
+    if (a.n_plast && !a.stdp_early) stdp_own<BF16, false>(a, rows, rec_t, s_act, &s_nact);
+    // Dense pulls into slot t + 1: the warp's groups of 128 entries, eight
+    // tested before their deliveries.
+    for (uint32_t c0 = wib; c0 < held * (kQ / 32u); c0 += 8u * kWarps) {
+      uint32_t hit = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < 8u; ++k) {
+        const uint32_t c = c0 + k * kWarps;
+        if (c < held * (kQ / 32u)) hit |= test4(rows, s_ent[c * 32u + lane]) << (4u * k);
+      }
+      while (hit) {
+        const uint32_t k = (__ffs(hit) - 1u) >> 2;
+        deliver((c0 + k * kWarps) * 32u + lane, (hit >> (4u * k)) & 15u, ix.slot);
+        hit &= ~(15u << (4u * k));
+      }
+    }
+    for (uint32_t c = held * (kQ / 32u) + wib; c < mine * (kQ / 32u); c += kWarps)
+      deliver(c * 32u + lane, test4(rows, entries(c * 32u + lane)), ix.slot);
+    push(ix, par);
+    grid_arrive(a, target);
+    if (s + 2u < n_steps) in_next = draw(ix.t + 1ull);
+    if (more && a.n_plast && a.stdp_early) {
+      // Rows as step t + 1 sees them: its offsets start one row further on.
+      stdp_own<BF16, true>(a, HistRows{s_hist, rows.base - a.n_words, row_words}, rec_t, s_act, &s_nact);
+    }
+    rows.base = rows.base == 0u ? row_words - a.n_words : rows.base - a.n_words;
+    if (!grid_wait(a, target, kPersistBlock - 32u)) aborted = true;
+  }
+  if (valid && lif) state_out(a, i, st);
+  if (a.recent && valid && n_steps) a.recent[((t0 + n_steps + 1ull) & 1ull) * a.n_pad + i] = reg;
+  if (a.raster_cap && blockIdx.x == 0) raster_offsets_from_counts(a, n_steps, s_wsum);
+  if (__ldcg(&ctl->error) & kErrBarrierTimeout) return;
+  hits = __reduce_add_sync(kFull, hits);
+  if (lane == 0 && walked) atomicAdd(&ctl->delivered, (unsigned long long)walked);
+  if (lane == 0 && hits) atomicAdd(&ctl->pulled, (unsigned long long)hits);
   if (leader) {
     ctl->step = t0 + n_steps;
     ctl->ring_slot = ix.slot;
@@ -2123,6 +2417,16 @@ cudaError_t launch_plast_reset(const StepArgs& a, int blocks, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Dynamic shared memory a kernel can take beside its static part.
+static size_t dyn_smem_max(const void* fn) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess || (size_t)optin <= fa.sharedSizeBytes) return 0;
+  return ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)255;
+}
+
 cudaError_t pull_setup() {
   const int mx = (int)kPullSumMax;
   cudaError_t e;
@@ -2142,6 +2446,9 @@ cudaError_t pull_setup() {
   if ((e = cudaFuncSetAttribute(k_persistent<false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))) return e;
   if ((e = cudaFuncSetAttribute(k_persistent_resident<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)))
     return e;
+  for (const void* fn : {(const void*)k_persistent_pull<true>, (const void*)k_persistent_pull<false>})
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem_max(fn))))
+      return e;
   return cudaFuncSetAttribute(k_persistent_resident<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
 }
 
@@ -2228,11 +2535,32 @@ int persistent_kernel_kind(const StepArgs& a, int blocks) {
   return a.n_pull_units == 0 ? SGB_KERNEL_FUSED : SGB_KERNEL_RESIDENT;
 }
 
+// Resident networks with dense pulls, one substep a step: k_persistent_pull,
+// when the history rows it keeps fit shared memory, no writer of row t + 1 can
+// meet a reader of row t (two rows), and the plastic windows, if any, come
+// from the spike registers.  Sets its dynamic shared memory (0: the two-barrier
+// form runs) and the pull units per block whose entries that holds.
+void plan_persistent_pull(StepArgs& a, int blocks) {
+  a.pull_smem = a.pull_held = 0;
+  if (blocks <= 0 || !a.n_pull_units || a.substeps != 1 || a.hist_rows < 2u || (a.n_plast && !a.recent3)) return;
+  const size_t most = dyn_smem_max(a.bf16 ? (const void*)k_persistent_pull<true>
+                                          : (const void*)k_persistent_pull<false>);
+  const size_t fixed = seg_smem_bytes(a) + (size_t)pull_rows(a) * a.n_words * 4;
+  if (fixed > most) return;
+  const uint32_t mine = (a.n_pull_units + (uint32_t)blocks - 1u) / (uint32_t)blocks;
+  a.pull_held = (uint32_t)std::min<size_t>(mine, (most - fixed) / (kPullUnit * 4));
+  a.pull_smem = (uint32_t)(fixed + (size_t)a.pull_held * kPullUnit * 4);
+}
+
 cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, cudaStream_t s) {
   StepArgs args = a;
   uint32_t n = n_steps;
   void* params[] = {&args, &n};
   const int kind = persistent_kernel_kind(a, blocks);
+  if (kind == SGB_KERNEL_RESIDENT && a.pull_smem)
+    return cudaLaunchCooperativeKernel(a.bf16 ? (const void*)k_persistent_pull<true>
+                                              : (const void*)k_persistent_pull<false>,
+                                       dim3(blocks), dim3(kPersistBlock), params, a.pull_smem, s);
   const bool resident = kind != SGB_KERNEL_GENERAL;
   const bool fused = kind == SGB_KERNEL_FUSED;
   const void* fn = fused      ? fused_kernel(a)
@@ -2253,16 +2581,9 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
 }
 
 uint32_t fused_row_smem_max() {
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  size_t st = 0;
-  for (const void* fn : kFusedKernels) {
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, fn);
-    st = fa.sharedSizeBytes > st ? fa.sharedSizeBytes : st;
-  }
-  return (size_t)optin > st ? (uint32_t)(((size_t)optin - st) & ~(size_t)255) : 0u;
+  size_t most = ~(size_t)0;
+  for (const void* fn : kFusedKernels) most = std::min(most, dyn_smem_max(fn));
+  return (uint32_t)most;
 }
 
 cudaError_t set_fused_row_smem(uint32_t bytes) {
