@@ -210,6 +210,8 @@ struct StepArgs {
   uint32_t item_cap;              // items per parity buffer
   uint32_t pull_smem;             // k_persistent_pull: dynamic shared memory (0: not run)
   uint32_t pull_held;             // its pull units per block with entries in shared memory
+  const uint32_t* pull_sorted;    // [n_pull_units][kPullUnit] its entries (k_pull_sort)
+  const uint4* pull_info;         // [n_pull_units] {projection, first entry, delay-1 entries, entries}
   uint32_t row_smem;              // fused persistent kernel: shared-memory bytes for push rows (0: none)
   uint32_t n_shards;              // fused persistent kernel: deferred shards (0: none)
   uint32_t shard_grid;            // the grid size the shards were dealt for
@@ -236,6 +238,8 @@ int persistent_blocks_per_sm(bool bf16);
 // Whether resident networks with dense pulls run k_persistent_pull, and its
 // shared memory (a.pull_smem, a.pull_held), for the handle's current modes.
 void plan_persistent_pull(StepArgs& a, int blocks);
+// Fills a.pull_sorted and a.pull_info (room for n_pull_units) from the dense tables.
+cudaError_t launch_pull_sort(const StepArgs& a, cudaStream_t s);
 // Dense pull (per-step driver): k_pull needs pull_setup() once per device
 // before its first launch.
 cudaError_t launch_pull(const StepArgs& a, int blocks, cudaStream_t s);

@@ -60,6 +60,7 @@ Sim::~Sim() {
   if (d_misc) cudaFree(d_misc);
   if (d_plast) cudaFree(d_plast);
   if (d_shard) cudaFree(d_shard);
+  if (d_sorted) cudaFree(d_sorted);
   if (ev_fork) cudaEventDestroy(ev_fork);
   if (ev_join) cudaEventDestroy(ev_join);
   if (side) cudaStreamDestroy(side);
@@ -257,6 +258,22 @@ static int upload_modes(Sim& s) {
   SGB_CUDA(cudaMemcpy((void*)a.projs, s.projs.data(), s.projs.size() * sizeof(ProjDev), cudaMemcpyHostToDevice));
   a.n_pull_units = (uint32_t)units.size();
   plan_persistent_pull(a, s.persistent_blocks);
+  if (a.pull_smem) {
+    // Its entries, sorted per unit: 4 B each and 16 B per unit, on the device.
+    const size_t need = (size_t)a.n_pull_units * (kPullUnit * 4 + sizeof(uint4));
+    if (need > s.sorted_bytes) {
+      if (s.d_sorted) cudaFree(s.d_sorted);
+      s.d_sorted = nullptr;
+      s.push_bytes -= s.sorted_bytes;
+      s.sorted_bytes = 0;
+      SGB_CUDA(cudaMalloc(&s.d_sorted, need));
+      s.sorted_bytes = need;
+      s.push_bytes += need;
+    }
+    a.pull_info = (const uint4*)s.d_sorted;
+    a.pull_sorted = (const uint32_t*)((char*)s.d_sorted + (size_t)a.n_pull_units * sizeof(uint4));
+    SGB_CUDA(launch_pull_sort(a, s.stream));
+  }
   // Fused persistent kernel.  Shards: the delay >= 3 parts of long rows
   // (longest first) are cut into kPushChunk-synapse shards dealt round-robin
   // over the blocks, so one spike's pushes spread over many SMs; a cell whose

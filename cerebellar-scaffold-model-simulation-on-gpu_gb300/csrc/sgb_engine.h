@@ -70,6 +70,8 @@ struct Sim {
   // Plasticity (STDP) of plastic projections.
   void* d_plast = nullptr;
   void* d_shard = nullptr;    // fused-kernel shards: split points, shard list, per-block offsets
+  void* d_sorted = nullptr;   // dense tables in the one-barrier resident kernel's form
+  size_t sorted_bytes = 0;
   size_t off_recent = 0;      // per-cell spike registers inside d_plast
   std::vector<PlastHost> plast;
   // Per-step drivers with early plasticity rules: k_stdp runs on `side`,

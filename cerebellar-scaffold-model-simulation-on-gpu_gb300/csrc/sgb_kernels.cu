@@ -653,15 +653,22 @@ __device__ __forceinline__ const uint32_t* hist_base(const StepArgs& a, uint32_t
 }
 
 template <bool BF16>
-__device__ __forceinline__ void pull_hit(const StepArgs& a, const ProjDev& P, uint32_t o,
-                                         uint32_t slot1) {
-  const uint32_t post = P.ell_rowmajor ? o / P.ell_K : o % P.post_count;
+__device__ __forceinline__ float pull_weight(const ProjDev& P, uint32_t o) {
   // A plastic projection's weights change every step (inside a persistent
   // launch too): read at L2, not through the non-coherent read-only path.
-  const float wv = BF16 ? __uint_as_float((uint32_t)__ldcg((const unsigned short*)P.ell_w + o) << 16)
-                        : __ldcg((const float*)P.ell_w + o);
-  const int v = __float2int_rn(wv);
-  atomicAdd(a.ring + (((size_t)slot1 * a.n_pad + P.post_base + post) << 1) + P.channel, v);
+  return BF16 ? __uint_as_float((uint32_t)__ldcg((const unsigned short*)P.ell_w + o) << 16)
+              : __ldcg((const float*)P.ell_w + o);
+}
+__device__ __forceinline__ size_t pull_target(const StepArgs& a, const ProjDev& P, uint32_t o,
+                                              uint32_t slot1) {
+  const uint32_t post = P.ell_rowmajor ? o / P.ell_K : o % P.post_count;
+  return (((size_t)slot1 * a.n_pad + P.post_base + post) << 1) + P.channel;
+}
+template <bool BF16>
+__device__ __forceinline__ void pull_hit(const StepArgs& a, const ProjDev& P, uint32_t o,
+                                         uint32_t slot1) {
+  const float wv = pull_weight<BF16>(P, o);
+  atomicAdd(a.ring + pull_target(a, P, o, slot1), __float2int_rn(wv));
 }
 
 // Persistent kernels: one of a unit's kPullParts ranges of kPullUnit /
@@ -986,6 +993,11 @@ __global__ void __launch_bounds__(kPullBlock, 1) k_pull_vec(StepArgs a) {
   if (lane == 0 && hits) atomicAdd(&a.ctl->pulled, (unsigned long long)hits);
 }
 
+// Block barrier 1 over the first n threads (a multiple of 32).
+__device__ __forceinline__ void bar_sync_first(uint32_t n) {
+  asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
+}
+
 // STDP of the plastic projections, step t (SynapticPlasticity.cu:40-120), run
 // after the cells of step t updated and before the dense pull that delivers
 // into slot t + 1, so that delivery uses the new values -- in the reference
@@ -1264,11 +1276,6 @@ __device__ __forceinline__ void grid_arrive_fenced(const StepArgs& a) {
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(a.bar) : "memory");
 }
 
-// Block barrier 1 over the first n threads (a multiple of 32).
-__device__ __forceinline__ void bar_sync_first(uint32_t n) {
-  asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory");
-}
-
 __device__ __forceinline__ bool grid_barrier(const StepArgs& a, unsigned long long& target) {
   grid_arrive(a, target);
   return grid_wait(a, target);
@@ -1292,7 +1299,7 @@ __host__ __device__ __forceinline__ uint32_t pull_rows(const StepArgs& a) {
 // scans them (all its threads call this; s_wsum holds kPersistBlock / 32).
 __device__ void raster_offsets_from_counts(const StepArgs& a, uint32_t n_steps, uint32_t* s_wsum) {
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-  const uint32_t per = (n_steps + kPersistBlock - 1) / kPersistBlock;
+  const uint32_t per = (n_steps + blockDim.x - 1) / blockDim.x;
   const uint32_t q0 = min(n_steps, threadIdx.x * per), q1 = min(n_steps, q0 + per);
   uint32_t tot = 0;
   for (uint32_t q = q0; q < q1; ++q)
@@ -1307,7 +1314,7 @@ __device__ void raster_offsets_from_counts(const StepArgs& a, uint32_t n_steps, 
   if (lane == 31) s_wsum[wib] = incl;
   __syncthreads();
   if (wib == 0) {
-    const uint32_t x = s_wsum[lane];
+    const uint32_t x = lane < (blockDim.x >> 5) ? s_wsum[lane] : 0u;
     uint32_t xi = x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1542,18 +1549,30 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_resident(StepAr
 // on its own bit, so only deliveries leave the SM: their weight and one
 // reduction.  The rows also free the writers of row t + 1 from readers of
 // row t + 1 - H.
+//   A unit's entries come sorted by spike bit (k_pull_sort), each with its place
+// in the unit.  32 consecutive ones cover a few words, so a lane settles a
+// group of 32 with one look at the rows' summary bits, and only the groups
+// that pass (one in five to ten) are tested entry by entry: 70 warp
+// instructions per 128 entries without this made the test, at five warps per
+// scheduler, the longest part of the step.  Sorted, the delay-1 entries are a
+// prefix of the unit.  Only
+// those wait for the spikes of step t; the others' deliveries into slot t + 2
+// come from spikes of steps <= t as well, so they are made behind iteration t's
+// barrier arrival, in the time the barrier takes (the launch's first step
+// finds those into its slot made by the prologue, the last one makes none, so
+// a launch ends as with the other kernels).
 //   Plastic projections: the block that pulls a unit also updates its weights,
 // so a block barrier orders the two.  Rules that read only earlier steps'
 // spikes (stdp_early) make the update of step t + 1 behind iteration t's
-// barrier arrival, the others that of step t before its pulls.  The spike
-// registers stay in their owners' registers and are published in three
-// buffers (step mod 3): behind the arrival, faster blocks already write those
-// of step t + 2 while step t's are read.
-//   What bounds it is latency: ring slot and history row (one L2 round trip),
-// the test of 18 entries a thread, weight, reduction, barrier.  92,550 cells,
-// every projection dense, 16-bit weights: 9.0 us per step with two barriers and
-// the entries read from L2 -> 4.6 us; Teacher rule on 1.75M synapses 10.2 ->
-// 6.1 us.
+// barrier arrival, the others that of step t before its pulls (and all of
+// them then).  The spike registers stay in their owners' registers and are
+// published in three buffers (step mod 3): behind the arrival, faster blocks
+// already write those of step t + 2 while step t's are read.
+//   What bounds it is latency: history row and ring slot (one L2 round trip),
+// the test of the delay-1 entries, weight, reduction, barrier.  92,550 cells:
+// every projection dense, 16-bit weights, 9.0 us per step with two barriers
+// and the entries read from L2 -> 4.1 us; Teacher rule on 1.75M synapses
+// 10.2 -> 5.1 us (one barrier alone, every entry tested: 4.5 and 6.0 us).
 struct HistRows {     // rows of the last steps, newest at word `base`, in decreasing step order
   const uint32_t* s;
   uint32_t base, total;  // total: words of all rows (the rows are a ring)
@@ -1566,69 +1585,166 @@ struct HistRows {     // rows of the last steps, newest at word `base`, in decre
   }
 };
 
-// The plasticity of a step on the block's own units (h and recent as the step
-// sees them): threads screen sub-units of kStdpUnit cells, then warps update the ones that can change.  The caller's
-// block barriers order it against the block's pulls; *s_n is 0 on entry.
-template <bool BF16, bool EARLY>
-__device__ __forceinline__ void stdp_own(const StepArgs& a, const HistRows& h,
-                                         const unsigned long long* recent, uint32_t* s_list,
-                                         uint32_t* s_n) {
-  constexpr uint32_t kSub = kPullUnit / kStdpUnit;
-  const uint32_t pad = a.hist_rows * a.n_pad;
-  const uint32_t mine = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x;
-  for (uint32_t b = 0; b < mine * kSub; b += kPersistBlock) {
-    const uint32_t x = b + threadIdx.x;
-    if (x < mine * kSub) {
-      const PullUnit pu = a.pull_units[blockIdx.x + (x / kSub) * gridDim.x];
-      const uint32_t o0 = pu.o0 + (x % kSub) * kStdpUnit;
-      for (uint32_t k = 0; k < a.n_plast; ++k) {
-        const PlastDev& L = a.plast[k];
-        const ProjDev& P = a.projs[L.proj];
-        if (L.proj != pu.proj || o0 >= P.ell_n) continue;
-        bool active = L.a0 != 0.f || L.a1_j != 0.f || !P.ell_rowmajor, one = false;
-        if (!active) {
-          const uint32_t p0 = o0 / P.ell_K, p1 = (min(o0 + kStdpUnit, P.ell_n) - 1u) / P.ell_K;
-          for (uint32_t p = p0; p <= p1; ++p) active |= stdp_post_spiked(L, P, h, p);
-          one = active && p0 == p1;
-        }
-        if (active) s_list[atomicAdd(s_n, 1u)] = threadIdx.x | (k << 16) | (one ? 1u << 31 : 0u);
+// A unit's entries in k_persistent_pull's form: the spike bit's word above the
+// step's row << 15 | place in the unit << 5 | bit in the word, ascending;
+// padding (word pull_rows * n_words, which the ring of rows maps to row 0)
+// last.  A group is 32 consecutive ones, one per lane.
+constexpr uint32_t kWordShift = 15;
+static_assert(kPullUnit == 1u << (kWordShift - 5), "place of an entry in its unit");
+constexpr uint32_t kGroup = 32, kGroups = kPullUnit / kGroup;
+
+// Units of a block and what each needs besides its entries.
+struct PullInfo {
+  uint32_t proj, o0;
+  uint32_t n1, n;  // delay-1 entries, entries (without padding)
+};
+static_assert(sizeof(PullInfo) == 16, "PullInfo copied as uint4");
+
+// Sorts the entries of unit blockIdx.x (bitonic, two entries per thread).
+__global__ void __launch_bounds__(kPullUnit / 2) k_pull_sort(StepArgs a, uint32_t* out, uint4* info) {
+  __shared__ uint32_t s[kPullUnit];
+  const PullUnit un = a.pull_units[blockIdx.x];
+  const uint32_t* src = a.projs[un.proj].ell_syn + un.o0;
+  const uint32_t pad = pull_rows(a) * a.n_pad;
+  uint32_t n1 = 0, n = 0;
+  for (uint32_t p = threadIdx.x; p < kPullUnit; p += kPullUnit / 2) {
+    const uint32_t e = min(src[p], pad);
+    s[p] = ((e >> 5) << kWordShift) | (p << 5) | (e & 31u);
+    n1 += (uint32_t)__syncthreads_count(e < a.n_pad);
+    n += (uint32_t)__syncthreads_count(e < pad);
+  }
+  for (uint32_t k = 2; k <= kPullUnit; k <<= 1)
+    for (uint32_t d = k >> 1; d; d >>= 1) {
+      __syncthreads();
+      const uint32_t x = ((threadIdx.x & ~(d - 1u)) << 1) | (threadIdx.x & (d - 1u)), y = x | d;
+      const uint32_t u = s[x], v = s[y];
+      if ((u > v) == ((x & k) == 0u)) {
+        s[x] = v;
+        s[y] = u;
       }
     }
-    __syncthreads();
-    const uint32_t n = *s_n;
-    for (uint32_t j = threadIdx.x >> 5; j < n; j += kPersistBlock / 32) {
-      const uint32_t v = s_list[j], y = b + (v & 0xFFFFu);
-      const uint32_t o0 = a.pull_units[blockIdx.x + (y / kSub) * gridDim.x].o0;
-      stdp_unit<BF16, true, EARLY>(a, PullUnit{(v >> 16) & 0x7FFFu, o0 + (y % kSub) * kStdpUnit}, h, pad,
-                                   recent, v >> 31);
+  __syncthreads();
+  for (uint32_t p = threadIdx.x; p < kPullUnit; p += kPullUnit / 2)
+    out[blockIdx.x * kPullUnit + p] = s[p];
+  if (threadIdx.x == 0) info[blockIdx.x] = make_uint4(un.proj, un.o0, n1, n);
+}
+
+// Units of the calling block, and the dynamic shared memory of k_persistent_pull:
+// segment descriptors and sources, projections, the history rows and a summary
+// bit per word of them, then per held unit its entries, its PullInfo, with
+// plastic projections where each sub-unit's post / teacher spikes are, its
+// groups' words and its groups in the two work lists.
+__host__ __device__ __forceinline__ size_t pull_proj_bytes(const StepArgs& a) {
+  return ((size_t)a.n_projs * sizeof(ProjDev) + 15) & ~(size_t)15;
+}
+__host__ __device__ __forceinline__ uint32_t pull_sum_words(const StepArgs& a) {
+  return (pull_rows(a) * a.n_swords + 1u + 3u) & ~3u;  // and one that a group's look may run into
+}
+__host__ __device__ __forceinline__ size_t pull_fixed_bytes(const StepArgs& a) {
+  return seg_smem_bytes_dev(a) + pull_proj_bytes(a) + (size_t)pull_rows(a) * a.n_words * 4 +
+         (size_t)pull_sum_words(a) * 4;
+}
+constexpr uint32_t kSub = kPullUnit / kStdpUnit;  // plasticity sub-units per pull unit
+__host__ __device__ __forceinline__ size_t pull_unit_bytes(const StepArgs& a) {
+  return kPullUnit * 4 + sizeof(PullInfo) + kGroups * (4 + 2 * 2) + (a.n_plast ? kSub * sizeof(uint2) : 0);
+}
+
+// Sub-unit x of the block (kStdpUnit ELL cells from *o0 of plastic projection
+// *k): where the spikes of its one or two posts (or their teachers) are above
+// the step's history row (.y kNever: one post), or kAlways in .y when every
+// cell may change or it covers more posts; kNever in .x: no spike, or not
+// plastic.
+constexpr uint32_t kAlways = 0xFFFFFFFEu, kNever = 0xFFFFFFFFu;
+__device__ __forceinline__ uint2 stdp_sub(const StepArgs& a, uint32_t x, uint32_t* k, uint32_t* o0) {
+  const PullUnit pu = a.pull_units[blockIdx.x + (x / kSub) * gridDim.x];
+  *o0 = pu.o0 + (x % kSub) * kStdpUnit;
+  for (*k = 0; *k < a.n_plast; ++*k) {
+    const PlastDev& L = a.plast[*k];
+    const ProjDev& P = a.projs[L.proj];
+    if (L.proj != pu.proj || *o0 >= P.ell_n) continue;
+    if (L.a0 != 0.f || L.a1_j != 0.f || !P.ell_rowmajor) return make_uint2(kAlways, kAlways);
+    const uint32_t p0 = *o0 / P.ell_K, p1 = (min(*o0 + kStdpUnit, P.ell_n) - 1u) / P.ell_K;
+    if (p1 > p0 + 1u) return make_uint2(kAlways, kAlways);
+    const bool te = L.rule == SGB_STDP_TEACHER;
+    const uint32_t s0 = te ? __ldg(L.teacher + p0) : P.post_base + p0;
+    if (p1 == p0) return make_uint2(s0, kNever);
+    const uint32_t s1 = te ? __ldg(L.teacher + p1) : P.post_base + p1;
+    return make_uint2(s0, s1 == kNever ? s0 : s1);  // a post without a teacher never changes
+  }
+  return make_uint2(kNever, kNever);
+}
+
+// The plasticity of a step on the block's own units (h and recent as the step
+// sees them): threads screen sub-units, then warps update those that can
+// change.  s_sub: the held sub-units' stdp_sub, or NULL.  Run by the block's
+// first n_thr threads, which meet on block barrier 1 (0 when all run it);
+// it ends with that barrier when anything was updated.  s_n[2] counts the
+// active sub-units of alternate rounds, par the next round's.
+template <bool BF16, bool EARLY>
+__device__ __forceinline__ void stdp_own(const StepArgs& a, const HistRows& h,
+                                         const unsigned long long* recent, const uint2* s_sub,
+                                         uint32_t* s_list, uint32_t* s_n, uint32_t& par, uint32_t n_thr) {
+  auto sync = [n_thr] {
+    if (n_thr == blockDim.x) __syncthreads(); else bar_sync_first(n_thr);
+  };
+  const uint32_t pad = a.hist_rows * a.n_pad;
+  const uint32_t n_sub = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x * kSub;
+  for (uint32_t b = 0; b < n_sub; b += n_thr, par ^= 1u) {
+    const uint32_t x = b + threadIdx.x;
+    if (x < n_sub) {
+      uint32_t k, o0;
+      const uint2 so = s_sub ? s_sub[x] : stdp_sub(a, x, &k, &o0);
+      bool active = so.y == kAlways;
+      if (!active) active = (so.x != kNever && h.bit(so.x)) || (so.y != kNever && h.bit(so.y));
+      if (active) s_list[atomicAdd(&s_n[par], 1u)] = threadIdx.x | (so.y == kNever ? 1u << 31 : 0u);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) *s_n = 0;
-    __syncthreads();
+    sync();
+    const uint32_t n = s_n[par];
+    if (threadIdx.x == 0) s_n[par ^ 1u] = 0;  // its readers were before this barrier
+    for (uint32_t j = threadIdx.x >> 5; j < n; j += n_thr >> 5) {
+      const uint32_t v = s_list[j];
+      uint32_t k, o0;
+      stdp_sub(a, b + (v & 0xFFFFu), &k, &o0);
+      stdp_unit<BF16, true, EARLY>(a, PullUnit{k, o0}, h, pad, recent, v >> 31);
+    }
+    if (n) sync();
   }
 }
 
-template <bool BF16>
-__global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a, uint32_t n_steps) {
-  // Dynamic shared memory: segment descriptors and sources, the history rows,
-  // then the entries of the block's first a.pull_held units.
+template <bool BF16, uint32_t MAXT>
+__global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_t n_steps) {
+  const uint32_t n_thr = blockDim.x, n_wrp = n_thr >> 5;  // pull_threads
   __shared__ uint2 s_items[kGenItems];
   __shared__ uint32_t s_icnt[2];
   __shared__ uint32_t s_wsum[kPersistBlock / 32];
   __shared__ uint32_t s_act[kPersistBlock];  // active plastic sub-units
-  __shared__ uint32_t s_nact;
+  __shared__ uint32_t s_nact[2], s_n1, s_n2;
+  __shared__ uint32_t s_od[kPersistBlock];  // out-degree of each thread's cell
+  __shared__ int s_ok;
   const uint32_t n_rows = pull_rows(a), row_words = n_rows * a.n_words;
-  uint32_t* s_hist = reinterpret_cast<uint32_t*>(g_dyn + seg_smem_bytes_dev(a));
-  uint4* s_ent = reinterpret_cast<uint4*>(s_hist + row_words);
+  const uint32_t mine = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x;
+  const uint32_t held = min(mine, a.pull_held);
+  ProjDev* s_proj = reinterpret_cast<ProjDev*>(g_dyn + seg_smem_bytes_dev(a));
+  uint32_t* s_hist = reinterpret_cast<uint32_t*>(g_dyn + seg_smem_bytes_dev(a) + pull_proj_bytes(a));
+  uint32_t* s_sum = s_hist + row_words;  // bit w: word w of the rows is not 0
+  uint32_t* s_ent = s_sum + pull_sum_words(a);
+  PullInfo* s_info = reinterpret_cast<PullInfo*>(s_ent + (size_t)held * kPullUnit);
+  uint2* s_sub = reinterpret_cast<uint2*>(s_info + held);
+  uint32_t* s_rng = reinterpret_cast<uint32_t*>(s_sub + (a.n_plast ? held * kSub : 0u));
+  uint16_t* s_g1 = reinterpret_cast<uint16_t*>(s_rng + held * kGroups);
+  uint16_t* s_g2 = s_g1 + held * kGroups;  // groups with delay-1 entries; with later ones
   {
     const uint4* src = reinterpret_cast<const uint4*>(a.segs);
     uint4* dst = reinterpret_cast<uint4*>(g_dyn);
-    for (uint32_t j = threadIdx.x; j < a.n_segs * (uint32_t)(sizeof(SegDev) / 16); j += kPersistBlock)
+    for (uint32_t j = threadIdx.x; j < a.n_segs * (uint32_t)(sizeof(SegDev) / 16); j += n_thr)
       dst[j] = src[j];
     const uint2* ss = reinterpret_cast<const uint2*>(a.srcs);
     uint2* sd = reinterpret_cast<uint2*>(g_dyn + seg_table_bytes(a.n_segs));
-    for (uint32_t j = threadIdx.x; j < a.n_srcs * (uint32_t)(sizeof(SrcDev) / 8); j += kPersistBlock)
+    for (uint32_t j = threadIdx.x; j < a.n_srcs * (uint32_t)(sizeof(SrcDev) / 8); j += n_thr)
       sd[j] = ss[j];
+    const uint2* ps = reinterpret_cast<const uint2*>(a.projs);
+    for (uint32_t j = threadIdx.x; j < a.n_projs * (uint32_t)(sizeof(ProjDev) / 8); j += n_thr)
+      reinterpret_cast<uint2*>(s_proj)[j] = ps[j];
   }
   const SegDev* segs = reinterpret_cast<const SegDev*>(g_dyn);
   const SrcDev* srcs = reinterpret_cast<const SrcDev*>(g_dyn + seg_table_bytes(a.n_segs));
@@ -1636,54 +1752,67 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a
   StepIdx ix = step_of(a);
   const unsigned long long t0 = ix.t;
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-  constexpr uint32_t kWarps = kPersistBlock / 32;
   const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
+  // A rule that reads the step's own spikes changes weights between a step's
+  // publication and its pulls, so then no pull goes ahead.
+  const bool ahead = a.n_plast == 0u || a.stdp_early != 0u;
+  if (threadIdx.x == 0) s_icnt[0] = s_icnt[1] = s_nact[0] = s_nact[1] = s_n1 = s_n2 = 0;
   // The rows of steps t0 - 1, t0 - 2, ...; row 0 (step t0) follows in the loop.
-  for (uint32_t j = a.n_words / 4u + threadIdx.x; j < row_words / 4u; j += kPersistBlock)
+  for (uint32_t j = a.n_words / 4u + threadIdx.x; j < row_words / 4u; j += n_thr)
     reinterpret_cast<uint4*>(s_hist)[j] = __ldcg(reinterpret_cast<const uint4*>(hist_base(a, ix.hrow)) + j);
-  // Entries; padding becomes pad1, which the ring of rows maps to row 0.
-  const uint32_t pad = a.hist_rows * a.n_pad, pad1 = n_rows * a.n_pad;
-  const uint32_t mine = (a.n_pull_units + gridDim.x - 1u - blockIdx.x) / gridDim.x;
-  const uint32_t held = min(mine, a.pull_held);
-  constexpr uint32_t kQ = kPullUnit / 4;  // 16-byte groups per unit
-  auto entries = [&](uint32_t q) -> uint4 {  // group q of the block's units, padding as pad1
-    const PullUnit un = a.pull_units[blockIdx.x + (q / kQ) * gridDim.x];
-    uint4 e = __ldg(reinterpret_cast<const uint4*>(a.projs[un.proj].ell_syn + un.o0) + q % kQ);
-    e.x = min(e.x, pad1); e.y = min(e.y, pad1); e.z = min(e.z, pad1); e.w = min(e.w, pad1);
-    return e;
-  };
-  for (uint32_t q = threadIdx.x; q < held * kQ; q += kPersistBlock) s_ent[q] = entries(q);
+  for (uint32_t j = threadIdx.x; j < pull_sum_words(a); j += n_thr) s_sum[j] = 0u;
+  constexpr uint32_t kQ = kPullUnit / 4;  // 16-byte loads per unit
+  const uint4* ents = reinterpret_cast<const uint4*>(a.pull_sorted);
+  const uint32_t n_held = held * kGroups, n_mine = mine * kGroups;  // groups
+  for (uint32_t q = threadIdx.x; q < held * kQ; q += n_thr)
+    reinterpret_cast<uint4*>(s_ent)[q] = __ldg(ents + (size_t)(blockIdx.x + (q / kQ) * gridDim.x) * kQ + q % kQ);
+  for (uint32_t k = threadIdx.x; k < held; k += n_thr)
+    reinterpret_cast<uint4*>(s_info)[k] = __ldg(a.pull_info + blockIdx.x + k * gridDim.x);
+  if (a.n_plast)
+    for (uint32_t x = threadIdx.x; x < held * kSub; x += n_thr) {
+      uint32_t k, o0;
+      s_sub[x] = stdp_sub(a, x, &k, &o0);
+    }
+  const uint2* subs = a.n_plast && held == mine ? s_sub : nullptr;
+  __syncthreads();
+  for (uint32_t j = a.n_words + threadIdx.x; j < row_words; j += n_thr)
+    if (s_hist[j]) atomicOr(s_sum + (j >> 5), 1u << (j & 31u));
+  // A group's words: first << 6 | span, span 0 for more than 32 words or
+  // several rows, where every lane looks its own word up.
+  for (uint32_t x = threadIdx.x; x < n_held; x += n_thr) {
+    const PullInfo& f = s_info[x / kGroups];
+    const uint32_t g = x % kGroups * kGroup, n1 = ahead ? f.n1 : f.n;
+    const uint32_t w0 = s_ent[x * kGroup] >> kWordShift, w1 = s_ent[x * kGroup + kGroup - 1u] >> kWordShift;
+    s_rng[x] = (w0 << 6) | (w0 / a.n_words == w1 / a.n_words && w1 - w0 < 32u ? w1 - w0 + 1u : 0u);
+    if (g < n1) s_g1[atomicAdd(&s_n1, 1u)] = (uint16_t)x;
+    if (g + kGroup > n1 && g < f.n) s_g2[atomicAdd(&s_n2, 1u)] = (uint16_t)x;
+  }
   // Words are dealt round-robin over the blocks (word slot = warp x blocks + block).
   const uint32_t ws = wib * gridDim.x + blockIdx.x;
   const bool has = ws < a.n_upd_words;
-  uint32_t w = 0, seg = 0, i = 0, local = 0, mask = 0, r0 = 0, r1 = 0, od = 0;
-  bool valid = false, lif = false;
+  uint32_t w = 0, seg = 0, i = 0;
+  bool valid = false, lif = false, stim = false;
+  s_od[threadIdx.x] = 0;
   float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
+  unsigned long long reg = 0;  // the cell's spike register, bit j = step t - j
   if (has) {
     w = __ldg(a.upd_words + ws);
     seg = __ldg(a.seg_of_word + w);
     i = (w << 5) + lane;
     const SegDev& sd = a.segs[seg];
-    local = i - sd.base;
-    valid = local < sd.count;
+    valid = i - sd.base < sd.count;
     lif = sd.kind == kSegLif;
     if (valid) {
-      if (lif) st = state_in(a.su[i], a.sg[i], sd.Vr); else mask = __ldg(a.src_mask + i);
-      od = __ldg(a.outdeg + i);
-      if (a.any_push) {
-        r0 = __ldg(a.push_row + i);
-        r1 = __ldg(a.push_row + i + 1);
-      }
+      if (lif) st = state_in(a.su[i], a.sg[i], sd.Vr); else stim = __ldg(a.src_mask + i) != 0u;
+      s_od[threadIdx.x] = __ldg(a.outdeg + i);
+      if (a.recent) reg = a.recent[((t0 + 1ull) & 1ull) * a.n_pad + i];
     }
   }
-  if (threadIdx.x == 0) s_icnt[0] = s_icnt[1] = s_nact = 0;
   __syncthreads();
-  const bool stim = mask != 0u, rd = lif && valid;
+  const bool rd = lif && valid;
   unsigned long long target = 0;
   uint32_t walked = 0, hits = 0;
   int2* ring2 = reinterpret_cast<int2*>(a.ring);
-  unsigned long long reg = 0;  // the cell's spike register, bit j = step t - j
-  if (a.recent && valid) reg = a.recent[((t0 + 1ull) & 1ull) * a.n_pad + i];
   uint32_t tri = (uint32_t)(t0 % 3ull);  // buffer of the last published step
   // Publishes the spikes of step px.t (chunk row px.rel): bitmap, counts,
   // spike register, and push items of parity par.
@@ -1693,44 +1822,88 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a
       reg = (reg << 1) | (fired ? 1ull : 0ull);
       a.recent3[(size_t)tri * a.n_pad + i] = reg;
     }
-    walked += publish_word<BF16, true>(a, w, seg, i, fired, r0, r1, od, px,
+    uint32_t r0 = 0, r1 = 0;
+    if (fired && a.any_push) {
+      r0 = __ldg(a.push_row + i);
+      r1 = __ldg(a.push_row + i + 1);
+    }
+    walked += publish_word<BF16, true>(a, w, seg, i, fired, r0, r1, s_od[threadIdx.x], px,
                                        BlockItems{s_items, &s_icnt[par]});
   };
   auto push = [&](const StepIdx& px, uint32_t par) {  // after a block barrier
     const uint32_t n_items = min(s_icnt[par], kGenItems);
     if (threadIdx.x == 0) s_icnt[par ^ 1u] = 0;
-    for (uint32_t u = wib; u < n_items; u += kWarps) walked += push_item<BF16>(a, s_items[u], px.slot);
+    for (uint32_t u = wib; u < n_items; u += n_wrp) walked += push_item<BF16>(a, s_items[u], px.slot);
   };
-  // Deliveries of one lane's hits in group q: bit j of `hit` is entry j.
-  auto deliver = [&](uint32_t q, uint32_t hit, uint32_t slot1) {
-    const PullUnit un = a.pull_units[blockIdx.x + (q / kQ) * gridDim.x];
-    const ProjDev& P = a.projs[un.proj];
-    while (hit) {
-      const uint32_t j = __ffs(hit) - 1u;
-      hit &= hit - 1u;
-      ++hits;
-      pull_hit<BF16>(a, P, un.o0 + (q % kQ) * 4u + j, slot1);
+  const uint32_t split = ahead ? a.n_words : row_words;
+  // Whether one of the group's words is set (one group per lane).
+  auto may_hit = [&](const HistRows& h, uint32_t rng) -> bool {
+    const uint32_t span = rng & 63u;
+    uint32_t x = h.base + (rng >> 6);
+    x = min(x, x - h.total);
+    const uint32_t* p = s_sum + (x >> 5);
+    return span == 0u || (__funnelshift_r(p[0], p[1], x) & (0xFFFFFFFFu >> (32u - span))) != 0u;
+  };
+  // Delivery of the lane's entry e of a unit, if its bit is set and its word is
+  // in [lo, hi) (padding lies beyond).  The first one waits in (pend_a,
+  // pend_w) with its weight's load in flight until flush().
+  uint32_t pend_a = kNever;
+  float pend_w = 0.f;
+  auto test = [&](const HistRows& h, uint32_t e, uint32_t lo, uint32_t hi) -> bool {
+    const uint32_t w = e >> kWordShift;
+    return ((h.word(w) >> (e & 31u)) & 1u) != 0u && w - lo < hi - lo;
+  };
+  auto hit = [&](const PullInfo& f, uint32_t e, uint32_t slot) {
+    ++hits;
+    const uint32_t o = f.o0 + ((e >> 5) & (kPullUnit - 1u));
+    const ProjDev& P = s_proj[f.proj];
+    if (pend_a == kNever) {
+      pend_w = pull_weight<BF16>(P, o);
+      pend_a = (uint32_t)pull_target(a, P, o, slot);
+    } else {
+      pull_hit<BF16>(a, P, o, slot);
     }
   };
-  auto test4 = [&](const HistRows& h, uint4 e) -> uint32_t {
-    const uint32_t v = h.bit(e.x) | (h.bit(e.y) << 1) | (h.bit(e.z) << 2) | (h.bit(e.w) << 3);
-    // A padding entry reads some bit of row 0; it is told apart only on a hit.
-    return v == 0u ? 0u
-                   : v & ((e.x < pad1 ? 1u : 0u) | (e.y < pad1 ? 2u : 0u) | (e.z < pad1 ? 4u : 0u) |
-                          (e.w < pad1 ? 8u : 0u));
+  // A warp's share (of n_w warps) of a work list: a group per lane against the
+  // summaries, then the few that pass, an entry per lane.
+  auto pull = [&](const HistRows& h, const uint16_t* list, uint32_t n, uint32_t lo, uint32_t hi,
+                  uint32_t slot, uint32_t n_w) {
+    for (uint32_t c0 = wib; c0 < n; c0 += 32u * n_w) {
+      const uint32_t c = c0 + lane * n_w;
+      const uint32_t x = c < n ? list[c] : 0u;
+      uint32_t todo = __ballot_sync(kFull, c < n && may_hit(h, s_rng[x]));
+      while (todo) {
+        const uint32_t g = __shfl_sync(kFull, x, __ffs(todo) - 1);
+        todo &= todo - 1u;
+        const uint32_t e = s_ent[g * kGroup + lane];
+        if (test(h, e, lo, hi)) hit(s_info[g / kGroups], e, slot);
+      }
+    }
+  };
+  auto flush = [&]() {
+    if (pend_a != kNever) atomicAdd(a.ring + pend_a, __float2int_rn(pend_w));
+    pend_a = kNever;
   };
   const auto draw = [&](unsigned long long t) {
-    return stim && input_fire(a, srcs, segs[seg], local, mask, t);
+    return stim && input_fire(a, srcs, segs[seg], i - segs[seg].base, __ldg(a.src_mask + i), t);
   };
   HistRows rows{s_hist, 0u, row_words};  // newest row: step t
+  uint32_t act_par = 0;
   bool in_next = false, aborted = false;
   if (n_steps) {
     if (a.n_plast && a.stdp_early)
-      stdp_own<BF16, true>(a, rows, a.recent + ((t0 + 1ull) & 1ull) * a.n_pad, s_act, &s_nact);
+      stdp_own<BF16, true>(a, rows, a.recent + ((t0 + 1ull) & 1ull) * a.n_pad, subs, s_act, s_nact,
+                           act_par, n_thr);
     ix.rel = 0;
-    clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
+    clear_next_summary(a, ix, blockIdx.x * n_thr + threadIdx.x, gridDim.x * n_thr);
     publish(valid && (lif ? st.x > segs[seg].Vth : draw(t0)), ix, 0u);
     __syncthreads();
+    if (ahead) {
+      // The later delays' deliveries into slot t0 + 1, from steps before t0.
+      const uint32_t slot1 = ix.slot + 1u == a.ring_slots ? 0u : ix.slot + 1u;
+      pull(rows, s_g2, s_n2, split, row_words, slot1, n_wrp);
+      flush();
+    }
     push(ix, 0u);
     grid_arrive(a, target);
     if (n_steps > 1) in_next = draw(t0 + 1ull);
@@ -1746,16 +1919,22 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a
     if (threadIdx.x < n4) hv = __ldcg(src + threadIdx.x);
     int2 acc = make_int2(0, 0);
     if (rd) acc = __ldcg(ring2 + (ix.roff + i));
+    flush();  // delivered behind the last arrival, read from step t + 1 on
     const uint32_t consumed = ix.roff;
-    for (uint32_t j = kPersistBlock + threadIdx.x; j < n4; j += kPersistBlock) dst[j] = __ldcg(src + j);
-    if (threadIdx.x < n4) dst[threadIdx.x] = hv;
+    auto store = [&](uint32_t j, uint4 v) {  // four words of the row and their summary bits
+      dst[j] = v;
+      const uint32_t b = (v.x ? 1u : 0u) | (v.y ? 2u : 0u) | (v.z ? 4u : 0u) | (v.w ? 8u : 0u);
+      if (b) atomicOr(s_sum + (rows.base >> 5) + (j >> 3), b << ((4u * j) & 31u));
+    };
+    for (uint32_t j = n_thr + threadIdx.x; j < n4; j += n_thr) store(j, __ldcg(src + j));
+    if (threadIdx.x < n4) store(threadIdx.x, hv);
     // From here on ix is step t + 1, whose spikes this step publishes.
     ix.t += 1ull;
     ix.rel = s + 1u;
     ix_advance(a, ix);
-    clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
     const unsigned long long* rec_t = a.recent3 + (size_t)tri * a.n_pad;  // registers of step t
     if (more) tri = tri == 2u ? 0u : tri + 1u;
+    clear_next_summary(a, ix, blockIdx.x * n_thr + threadIdx.x, gridDim.x * n_thr);
     bool fired = in_next;
     if (has && lif) {
       const LifK k = lif_k(segs[seg]);
@@ -1766,33 +1945,51 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_pull(StepArgs a
     const uint32_t par = (s + 1u) & 1u;
     if (more) publish(fired, ix, par);
     __syncthreads();
-    if (a.n_plast && !a.stdp_early) stdp_own<BF16, false>(a, rows, rec_t, s_act, &s_nact);
-    // Dense pulls into slot t + 1: the warp's groups of 128 entries, eight
-    // tested before their deliveries.
-    for (uint32_t c0 = wib; c0 < held * (kQ / 32u); c0 += 8u * kWarps) {
-      uint32_t hit = 0;
-#pragma unroll
-      for (uint32_t k = 0; k < 8u; ++k) {
-        const uint32_t c = c0 + k * kWarps;
-        if (c < held * (kQ / 32u)) hit |= test4(rows, s_ent[c * 32u + lane]) << (4u * k);
-      }
-      while (hit) {
-        const uint32_t k = (__ffs(hit) - 1u) >> 2;
-        deliver((c0 + k * kWarps) * 32u + lane, (hit >> (4u * k)) & 15u, ix.slot);
-        hit &= ~(15u << (4u * k));
+    if (a.n_plast && !a.stdp_early)
+      stdp_own<BF16, false>(a, rows, rec_t, subs, s_act, s_nact, act_par, n_thr);
+    // Deliveries into slot t + 1: the delay-1 entries (every entry, when none
+    // goes ahead, and of the units that are not held).
+    pull(rows, s_g1, s_n1, 0u, split, ix.slot, n_wrp);
+    for (uint32_t c = n_held + wib; c < n_mine; c += n_wrp) {
+      const uint32_t u = blockIdx.x + (c / kGroups) * gridDim.x;
+      const uint32_t e = __ldg(a.pull_sorted + (size_t)u * kPullUnit + (c % kGroups) * kGroup + lane);
+      if (test(rows, e, 0u, row_words)) {
+        const uint4 f = __ldg(a.pull_info + u);
+        hit(PullInfo{f.x, f.y, f.z, f.w}, e, ix.slot);
       }
     }
-    for (uint32_t c = held * (kQ / 32u) + wib; c < mine * (kQ / 32u); c += kWarps)
-      deliver(c * 32u + lane, test4(rows, entries(c * 32u + lane)), ix.slot);
-    push(ix, par);
-    grid_arrive(a, target);
+    flush();
+    if (a.any_push) {
+      __syncthreads();
+      push(ix, par);
+    }
+    // The last warp arrives, its release waiting for the block's writes, and
+    // polls; the others go on.
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == n_thr - 32u)
+      asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(a.bar) : "memory");
     if (s + 2u < n_steps) in_next = draw(ix.t + 1ull);
-    if (more && a.n_plast && a.stdp_early) {
-      // Rows as step t + 1 sees them: its offsets start one row further on.
-      stdp_own<BF16, true>(a, HistRows{s_hist, rows.base - a.n_words, row_words}, rec_t, s_act, &s_nact);
+    if (wib == n_wrp - 1u) {
+      if (lane == 0) s_ok = poll_arrivals(a, target);
+      __syncwarp();
+    } else if (more && ahead) {
+      // As step t + 1 sees the rows: its offsets of a delay of 1 fall on the row
+      // that it is going to load (a group's test reads it, and drops the result).
+      const HistRows next{s_hist, rows.base == 0u ? row_words - a.n_words : rows.base - a.n_words,
+                          row_words};
+      if (a.n_plast)
+        stdp_own<BF16, true>(a, next, rec_t, subs, s_act, s_nact, act_par, n_thr - 32u);
+      const uint32_t slot2 = ix.slot + 1u == a.ring_slots ? 0u : ix.slot + 1u;
+      pull(next, s_g2, s_n2, split, row_words, slot2, n_wrp - 1u);
     }
     rows.base = rows.base == 0u ? row_words - a.n_words : rows.base - a.n_words;
-    if (!grid_wait(a, target, kPersistBlock - 32u)) aborted = true;
+    // The summary of the row that the next step replaces; the pulls made just
+    // above may still test it for groups that also hold later rows' entries, and
+    // drop what it says.
+    for (uint32_t j = threadIdx.x; j < a.n_swords; j += n_thr) s_sum[(rows.base >> 5) + j] = 0u;
+    __syncthreads();
+    aborted = !s_ok;
   }
   if (valid && lif) state_out(a, i, st);
   if (a.recent && valid && n_steps) a.recent[((t0 + n_steps + 1ull) & 1ull) * a.n_pad + i] = reg;
@@ -2417,6 +2614,23 @@ cudaError_t launch_plast_reset(const StepArgs& a, int blocks, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// k_persistent_pull by [BF16][block size up to kPullSmall or any]: with at most
+// 24 warps its threads may have 80 registers, so that nothing spills.
+// A warp for each of the block's words and one that keeps the grid barrier, at
+// least kPullWarps for the entries (16 warps: 2 % slower, 32 with 64
+// registers: 7 %).
+constexpr uint32_t kPullSmall = 768, kPullWarps = 24;
+static const void* const kPullKernels[] = {
+    (const void*)k_persistent_pull<false, kPullSmall>, (const void*)k_persistent_pull<false, kPersistBlock>,
+    (const void*)k_persistent_pull<true, kPullSmall>, (const void*)k_persistent_pull<true, kPersistBlock>};
+static uint32_t pull_threads(const StepArgs& a, int blocks) {
+  const uint32_t words = (a.n_upd_words + (uint32_t)blocks - 1u) / (uint32_t)blocks;
+  return 32u * std::min(std::max(words + 1u, kPullWarps), (uint32_t)kPersistBlock / 32u);
+}
+static const void* pull_kernel(const StepArgs& a, int blocks) {
+  return kPullKernels[(a.bf16 ? 2 : 0) + (pull_threads(a, blocks) > kPullSmall ? 1 : 0)];
+}
+
 // Dynamic shared memory a kernel can take beside its static part.
 static size_t dyn_smem_max(const void* fn) {
   int dev = 0, optin = 0;
@@ -2446,7 +2660,7 @@ cudaError_t pull_setup() {
   if ((e = cudaFuncSetAttribute(k_persistent<false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))) return e;
   if ((e = cudaFuncSetAttribute(k_persistent_resident<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)))
     return e;
-  for (const void* fn : {(const void*)k_persistent_pull<true>, (const void*)k_persistent_pull<false>})
+  for (const void* fn : kPullKernels)
     if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem_max(fn))))
       return e;
   return cudaFuncSetAttribute(k_persistent_resident<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
@@ -2543,13 +2757,20 @@ int persistent_kernel_kind(const StepArgs& a, int blocks) {
 void plan_persistent_pull(StepArgs& a, int blocks) {
   a.pull_smem = a.pull_held = 0;
   if (blocks <= 0 || !a.n_pull_units || a.substeps != 1 || a.hist_rows < 2u || (a.n_plast && !a.recent3)) return;
-  const size_t most = dyn_smem_max(a.bf16 ? (const void*)k_persistent_pull<true>
-                                          : (const void*)k_persistent_pull<false>);
-  const size_t fixed = seg_smem_bytes(a) + (size_t)pull_rows(a) * a.n_words * 4;
-  if (fixed > most) return;
+  if (persistent_kernel_kind(a, blocks) != SGB_KERNEL_RESIDENT) return;
+  const size_t most = dyn_smem_max(pull_kernel(a, blocks));
+  const size_t fixed = pull_fixed_bytes(a);
+  // The word of an entry's spike bit shares 32 bits with its place in the unit.
+  if (fixed > most || pull_rows(a) * a.n_words >= 1u << (32 - kWordShift)) return;
   const uint32_t mine = (a.n_pull_units + (uint32_t)blocks - 1u) / (uint32_t)blocks;
-  a.pull_held = (uint32_t)std::min<size_t>(mine, (most - fixed) / (kPullUnit * 4));
-  a.pull_smem = (uint32_t)(fixed + (size_t)a.pull_held * kPullUnit * 4);
+  a.pull_held = (uint32_t)std::min<size_t>(mine, (most - fixed) / pull_unit_bytes(a));
+  a.pull_smem = (uint32_t)(fixed + (size_t)a.pull_held * pull_unit_bytes(a));
+}
+
+cudaError_t launch_pull_sort(const StepArgs& a, cudaStream_t s) {
+  k_pull_sort<<<a.n_pull_units, kPullUnit / 2, 0, s>>>(a, const_cast<uint32_t*>(a.pull_sorted),
+                                                       const_cast<uint4*>(a.pull_info));
+  return cudaGetLastError();
 }
 
 cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, cudaStream_t s) {
@@ -2558,9 +2779,8 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
   void* params[] = {&args, &n};
   const int kind = persistent_kernel_kind(a, blocks);
   if (kind == SGB_KERNEL_RESIDENT && a.pull_smem)
-    return cudaLaunchCooperativeKernel(a.bf16 ? (const void*)k_persistent_pull<true>
-                                              : (const void*)k_persistent_pull<false>,
-                                       dim3(blocks), dim3(kPersistBlock), params, a.pull_smem, s);
+    return cudaLaunchCooperativeKernel(pull_kernel(a, blocks), dim3(blocks),
+                                       dim3(pull_threads(a, blocks)), params, a.pull_smem, s);
   const bool resident = kind != SGB_KERNEL_GENERAL;
   const bool fused = kind == SGB_KERNEL_FUSED;
   const void* fn = fused      ? fused_kernel(a)
