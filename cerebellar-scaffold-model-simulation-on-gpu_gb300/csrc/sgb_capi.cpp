@@ -319,7 +319,7 @@ int sgb_sim_get_info(const sgb_sim* sim, sgb_sim_info* info) {
                           ? persistent_kernel_kind(s.args, s.persistent_blocks)
                           : SGB_KERNEL_GRAPH;
   info->push_smem_bytes = info->step_kernel == SGB_KERNEL_FUSED ? (int32_t)s.args.row_smem : 0;
-  info->shard_cells = info->step_kernel == SGB_KERNEL_FUSED ? s.n_shard_cells : 0;
+  info->shard_cells = info->step_kernel == SGB_KERNEL_FUSED ? s.n_heavy_cells : 0;
   info->item_width = 1 << fused_item_log2(s.args);
   info->deliver_blocks = s.deliver_blocks;
   info->pull_summary = (int32_t)s.args.pull_sum;

@@ -39,12 +39,16 @@ namespace sgb {
 constexpr int kBlock = 256;           // threads per block of the per-step kernels
 constexpr int kPersistBlock = 1024;   // threads per block of the persistent kernel
 constexpr uint32_t kPushChunk = 256;  // synapses per push work item (8 per lane)
-// Fused persistent kernel: a cell with at least kShardMin synapses of delay
-// >= 3 keeps only its delay-1 and delay-2 synapses; the rest is cut into
-// shards of kPushChunk synapses that other blocks push one step later (two
-// in the late-push timeline; at most kMaxShards per block).
-constexpr uint32_t kShardMin = 256;
-constexpr uint32_t kMaxShards = 128;
+// Fused persistent kernel: 32-cell words that hold a row of at least kHeavyMin
+// synapses are delivered by the blocks of their targets (at most kHeavyWords).
+// One warp per block handles a step's heavy spikes one after another, so
+// exchange steps of several substeps, with as many times the spikes, leave
+// shorter rows to their own blocks (kHeavyMinSub; 97k cells, ten substeps,
+// rows of 147 synapses heavy 5.9 us per step, not heavy 4.6; one substep 1.71
+// and 1.91 us).
+constexpr uint32_t kHeavyMin = 128;
+constexpr uint32_t kHeavyMinSub = 256;
+constexpr uint32_t kHeavyWords = 128;
 constexpr uint32_t kPullUnit = 1024;  // ELL entries per dense-pull work unit (32 per lane)
 constexpr uint32_t kStdpUnit = 128;   // ELL cells per plasticity work unit (4 per lane)
 constexpr int kPullBlock = 1024;             // threads per k_pull block (one per SM)
@@ -187,7 +191,7 @@ struct StepArgs {
   uint32_t* raster;               // [raster_cap] padded ids
   uint32_t* raster_off;           // [chunk_steps + 1]
   double* totals;                 // [n_segs]
-  unsigned long long* bar;        // grid-barrier arrival counter (zeroed per launch)
+  unsigned long long* bar;        // grid-barrier arrival counter (zeroed per launch, with the board)
   uint32_t n_pad, n_words, n_segs, n_projs;
   uint32_t n_srcs;                // stimulus sources (all segments)
   uint32_t ring_slots, hist_rows;
@@ -213,11 +217,13 @@ struct StepArgs {
   const uint32_t* pull_sorted;    // [n_pull_units][kPullUnit] its entries (k_pull_sort)
   const uint4* pull_info;         // [n_pull_units] {projection, first entry, delay-1 entries, entries}
   uint32_t row_smem;              // fused persistent kernel: shared-memory bytes for push rows (0: none)
-  uint32_t n_shards;              // fused persistent kernel: deferred shards (0: none)
-  uint32_t shard_grid;            // the grid size the shards were dealt for
-  const uint32_t* push_split;     // [n_pad] end of the part of a row its owner pushes (shards on)
-  const uint4* shards;            // {cell, first synapse, length, 0}, grouped by block
-  const uint32_t* shard_off;      // [shard_grid + 1] each block's range of shards
+  // Heavy words of the fused persistent kernel, for a grid of hv_grid blocks.
+  uint32_t hv_words, hv_grid, hv_cap;  // words (0: none); most synapses of them onto one block
+  const uint32_t* push_split;     // [n_pad] end of the part of a row its block pushes
+  const uint16_t* hv_index;       // [n_words] index of a heavy word, 0xFFFF: not heavy
+  const uint16_t* hv_off;         // [hv_grid][hv_words * 32 + 1] first synapse of each heavy cell
+  const uint2* hv_syn;            // [hv_grid][hv_cap] {cell | delay << 10 | accumulator << 14, increment}
+  unsigned long long* board;      // [4][kHeavyWords] {step tag, spike bits}, zeroed per launch, after bar
   int32_t bf16;
   int32_t substeps;
 };
@@ -235,6 +241,8 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
 uint32_t fused_row_smem_max();
 cudaError_t set_fused_row_smem(uint32_t bytes);
 int persistent_blocks_per_sm(bool bf16);
+// Shared memory that the fused kernel's heavy words (a.hv_*) take on a grid of `blocks`.
+size_t fused_heavy_bytes(const StepArgs& a, int blocks);
 // Whether resident networks with dense pulls run k_persistent_pull, and its
 // shared memory (a.pull_smem, a.pull_held), for the handle's current modes.
 void plan_persistent_pull(StepArgs& a, int blocks);

@@ -31,6 +31,9 @@ namespace sgb {
                        __FILE__, __LINE__);                                                   \
   } while (0)
 
+// The grid barrier's counter has its memory line to itself; the board follows.
+constexpr size_t kBarBytes = 256;
+
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Access-policy window of the cell state on stream st (num_bytes 0 clears it).
@@ -59,7 +62,7 @@ Sim::~Sim() {
   if (d_push) cudaFree(d_push);
   if (d_misc) cudaFree(d_misc);
   if (d_plast) cudaFree(d_plast);
-  if (d_shard) cudaFree(d_shard);
+  if (d_heavy) cudaFree(d_heavy);
   if (d_sorted) cudaFree(d_sorted);
   if (ev_fork) cudaEventDestroy(ev_fork);
   if (ev_join) cudaEventDestroy(ev_join);
@@ -190,6 +193,93 @@ static bool build_ell(const Projection& pr, int32_t npost, uint32_t pre_base, ui
   return true;
 }
 
+// The fused kernel's heavy words: 32-cell words with a row of at least
+// kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
+// block has room for the words' synapses onto its cells (half of its shared
+// memory with the delay line; the push rows get the rest).  Fills the handle's
+// tables and takes the words' rows out of own_end (what a cell's block pushes).
+static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
+                        const std::vector<uint32_t>& syn, const std::vector<float>& wf,
+                        const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
+  StepArgs& a = s.args;
+  a.hv_words = a.hv_cap = a.hv_grid = 0;
+  s.n_heavy_cells = 0;
+  if (!fused) return SGB_OK;
+  const uint32_t B = (uint32_t)s.persistent_blocks;
+  std::vector<std::pair<uint64_t, uint32_t>> cand;  // {synapses, word}
+  const uint32_t least = a.substeps == 1 ? kHeavyMin : kHeavyMinSub;
+  for (uint32_t w : s.upd_words) {
+    uint32_t longest = 0;
+    for (uint32_t c = w * 32; c < w * 32 + 32; ++c) longest = std::max(longest, row[c + 1] - row[c]);
+    if (longest >= least) cand.push_back({(uint64_t)(row[w * 32 + 32] - row[w * 32]), w});
+  }
+  if (cand.empty()) return SGB_OK;
+  std::stable_sort(cand.begin(), cand.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::vector<uint32_t> slot_of_word(s.n_words, 0);
+  for (size_t ws = 0; ws < s.upd_words.size(); ++ws) slot_of_word[s.upd_words[ws]] = (uint32_t)ws;
+  auto target = [&](uint32_t q) { return slot_of_word[(syn[q] & kPushPostMask) >> 5]; };
+  const size_t budget = fused_row_smem_max() / 2;
+  std::vector<uint32_t> count(B, 0), add(B), words;
+  for (const auto& cw : cand) {
+    if (words.size() == kHeavyWords) break;
+    std::fill(add.begin(), add.end(), 0u);
+    for (uint32_t q = row[cw.second * 32]; q < row[cw.second * 32 + 32]; ++q) add[target(q) % B]++;
+    uint32_t most = 0;
+    for (uint32_t b = 0; b < B; ++b) most = std::max(most, count[b] + add[b]);
+    a.hv_words = (uint32_t)words.size() + 1;
+    a.hv_cap = most;
+    if (most > 0xFFFFu || fused_heavy_bytes(a, s.persistent_blocks) > budget) break;
+    for (uint32_t b = 0; b < B; ++b) count[b] += add[b];
+    words.push_back(cw.second);
+  }
+  a.hv_words = (uint32_t)words.size();
+  a.hv_cap = *std::max_element(count.begin(), count.end());
+  if (words.empty()) return SGB_OK;
+  const uint32_t n_off = a.hv_words * 32 + 1;
+  std::vector<uint16_t> index(s.n_words, 0xFFFF), off((size_t)B * n_off, 0);
+  std::vector<uint2> list((size_t)B * a.hv_cap, make_uint2(0, 0));
+  std::fill(count.begin(), count.end(), 0u);
+  for (uint32_t h = 0; h < a.hv_words; ++h) {
+    index[words[h]] = (uint16_t)h;
+    for (uint32_t j = 0; j < 32; ++j) {
+      const uint32_t c = words[h] * 32 + j;
+      for (uint32_t q = row[c]; q < row[c + 1]; ++q) {
+        const uint32_t ws = target(q), b = ws % B;
+        const uint32_t cell = (ws / B) * 32 + (syn[q] & 31u);  // within the block
+        const float v = s.bf16 ? bf16_bits_to_f32(wh[q]) : wf[q];
+        list[(size_t)b * a.hv_cap + count[b]++] =
+            make_uint2(cell | (((syn[q] >> kPushPostBits) & 15u) << 10) | ((syn[q] >> 31) << 14),
+                       (uint32_t)(int32_t)lrintf(v));
+      }
+      for (uint32_t b = 0; b < B; ++b) off[(size_t)b * n_off + h * 32 + j + 1] = (uint16_t)count[b];
+      if (row[c + 1] > row[c]) ++s.n_heavy_cells;
+      own_end[c] = row[c];
+    }
+  }
+  const size_t o_idx = align_up((size_t)s.n_pad * 4, 256), o_off = align_up(o_idx + index.size() * 2, 256);
+  const size_t o_syn = align_up(o_off + off.size() * 2, 256), need = o_syn + list.size() * sizeof(uint2);
+  if (need > s.heavy_bytes) {
+    if (s.d_heavy) cudaFree(s.d_heavy);
+    s.d_heavy = nullptr;
+    s.push_bytes -= s.heavy_bytes;
+    s.heavy_bytes = 0;
+    SGB_CUDA(cudaMalloc(&s.d_heavy, need));
+    s.heavy_bytes = need;
+    s.push_bytes += need;
+  }
+  char* hb = (char*)s.d_heavy;
+  SGB_CUDA(cudaMemcpy(hb, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
+  SGB_CUDA(cudaMemcpy(hb + o_idx, index.data(), index.size() * 2, cudaMemcpyHostToDevice));
+  SGB_CUDA(cudaMemcpy(hb + o_off, off.data(), off.size() * 2, cudaMemcpyHostToDevice));
+  SGB_CUDA(cudaMemcpy(hb + o_syn, list.data(), list.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  a.push_split = (const uint32_t*)hb;
+  a.hv_index = (const uint16_t*)(hb + o_idx);
+  a.hv_off = (const uint16_t*)(hb + o_off);
+  a.hv_syn = (const uint2*)(hb + o_syn);
+  a.hv_grid = B;
+  return SGB_OK;
+}
+
 // Rebuilds the merged push table (every projection in CSR mode, cell-major)
 // and the dense-pull work lists, uploads them, and drops captured graphs.
 static int upload_modes(Sim& s) {
@@ -210,28 +300,20 @@ static int upload_modes(Sim& s) {
   std::vector<uint32_t> syn((size_t)total);
   std::vector<float> wf(s.bf16 ? 0 : (size_t)total);
   std::vector<uint16_t> wh(s.bf16 ? (size_t)total : 0);
-  // Each row holds its delay-1 synapses first (pass 0), then its delay-2
-  // synapses (pass 1), then the others: split[c] is where the delay >= 3 part
-  // of cell c's row starts.
-  std::vector<uint32_t> split;
   {
     std::vector<uint32_t> fill(row.begin(), row.end() - 1);
-    for (int pass = 0; pass < 3; ++pass) {
-      for (size_t k = 0; k < s.projs.size(); ++k) {
-        if (s.projs[k].mode != SGB_PROP_CSR) continue;
-        const ProjTables& t = s.ptab[k];
-        const Projection& pr = s.nets[t.net].projs[t.proj];
-        const uint32_t pre_base = s.segs[t.pre_seg].base, post_base = s.segs[t.post_seg].base;
-        for (size_t i = 0; i < pr.pre_idx.size(); ++i) {
-          if (std::min<int>(pr.delay[i], 3) - 1 != pass) continue;
-          const uint32_t q = fill[pre_base + pr.pre_idx[i]]++;
-          syn[q] = (post_base + pr.post_idx[i]) | ((uint32_t)pr.delay[i] << kPushPostBits) |
-                   ((uint32_t)pr.channel << 31);
-          const float w = scaled_weight(pr.weight[i], t.scale_bits, s.bf16);
-          if (s.bf16) wh[q] = f32_to_bf16_bits(w); else wf[q] = w;
-        }
+    for (size_t k = 0; k < s.projs.size(); ++k) {
+      if (s.projs[k].mode != SGB_PROP_CSR) continue;
+      const ProjTables& t = s.ptab[k];
+      const Projection& pr = s.nets[t.net].projs[t.proj];
+      const uint32_t pre_base = s.segs[t.pre_seg].base, post_base = s.segs[t.post_seg].base;
+      for (size_t i = 0; i < pr.pre_idx.size(); ++i) {
+        const uint32_t q = fill[pre_base + pr.pre_idx[i]]++;
+        syn[q] = (post_base + pr.post_idx[i]) | ((uint32_t)pr.delay[i] << kPushPostBits) |
+                 ((uint32_t)pr.channel << 31);
+        const float w = scaled_weight(pr.weight[i], t.scale_bits, s.bf16);
+        if (s.bf16) wh[q] = f32_to_bf16_bits(w); else wf[q] = w;
       }
-      if (pass == 1) split = fill;
     }
   }
   const size_t wsz = s.bf16 ? 2 : 4;
@@ -274,74 +356,21 @@ static int upload_modes(Sim& s) {
     a.pull_sorted = (const uint32_t*)((char*)s.d_sorted + (size_t)a.n_pull_units * sizeof(uint4));
     SGB_CUDA(launch_pull_sort(a, s.stream));
   }
-  // Fused persistent kernel.  Shards: the delay >= 3 parts of long rows
-  // (longest first) are cut into kPushChunk-synapse shards dealt round-robin
-  // over the blocks, so one spike's pushes spread over many SMs; a cell whose
-  // shards no longer fit keeps its whole row.  Then shared memory for the
-  // push rows of the block holding the most synapses (word slot ws runs in
-  // block ws mod blocks; a sharded cell's own part is its delay-1 and delay-2
-  // synapses).
-  a.row_smem = 0;
-  a.n_shards = 0;
-  s.n_shard_cells = 0;
   const bool fused = total > 0 && s.persistent_blocks > 0 &&
                      persistent_kernel_kind(a, s.persistent_blocks) == SGB_KERNEL_FUSED;
+  a.row_smem = 0;
   std::vector<uint32_t> own_end(row.begin() + 1, row.end());
-  std::vector<std::vector<uint4>> blk_sh(fused && s.d_shard ? (size_t)s.persistent_blocks : 0);
-  if (!blk_sh.empty()) {
-    const uint32_t B = (uint32_t)blk_sh.size();
-    std::vector<uint32_t> cand;
-    for (uint32_t c = 0; c < s.n_pad; ++c)
-      if (row[c + 1] - split[c] >= kShardMin) cand.push_back(c);
-    std::stable_sort(cand.begin(), cand.end(), [&](uint32_t x, uint32_t y) {
-      return row[x + 1] - split[x] > row[y + 1] - split[y];
-    });
-    uint32_t cursor = 0;
-    for (uint32_t c : cand) {
-      std::vector<uint32_t> picked;
-      for (uint32_t q = split[c]; q < row[c + 1]; q += kPushChunk) {
-        uint32_t tries = 0;
-        while (tries < B && blk_sh[cursor].size() >= kMaxShards) { cursor = (cursor + 1) % B; ++tries; }
-        if (tries == B) break;
-        blk_sh[cursor].push_back(make_uint4(c, q, std::min(kPushChunk, row[c + 1] - q), 0u));
-        picked.push_back(cursor);
-        cursor = (cursor + 1) % B;
-      }
-      if ((uint64_t)picked.size() * kPushChunk < row[c + 1] - split[c]) {
-        for (uint32_t b : picked) blk_sh[b].pop_back();
-        break;
-      }
-      own_end[c] = split[c];
-      ++s.n_shard_cells;
-    }
-    std::vector<uint4> flat;
-    std::vector<uint32_t> off(B + 1, 0);
-    for (uint32_t b = 0; b < B; ++b) {
-      flat.insert(flat.end(), blk_sh[b].begin(), blk_sh[b].end());
-      off[b + 1] = (uint32_t)flat.size();
-    }
-    char* sb = (char*)s.d_shard;
-    const size_t o_sh = align_up((size_t)s.n_pad * 4, 256);
-    const size_t o_off = o_sh + align_up((size_t)B * kMaxShards * sizeof(uint4), 256);
-    SGB_CUDA(cudaMemcpy(sb, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
-    if (!flat.empty())
-      SGB_CUDA(cudaMemcpy(sb + o_sh, flat.data(), flat.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-    SGB_CUDA(cudaMemcpy(sb + o_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice));
-    a.push_split = (const uint32_t*)sb;
-    a.shards = (const uint4*)(sb + o_sh);
-    a.shard_off = (const uint32_t*)(sb + o_off);
-    a.shard_grid = B;
-    a.n_shards = (uint32_t)flat.size();
-  }
+  if (int rc = upload_heavy(s, fused, row, syn, wf, wh, own_end)) return rc;
   if (fused) {
+    // Shared memory for the push rows of the block holding the most synapses
+    // (word slot ws runs in block ws mod blocks), beside the heavy words'.
     std::vector<uint64_t> need((size_t)s.persistent_blocks, 0);
     for (size_t ws = 0; ws < s.upd_words.size(); ++ws) {
       const uint32_t w = s.upd_words[ws];
       for (uint32_t c = w * 32; c < w * 32 + 32; ++c) need[ws % need.size()] += own_end[c] - row[c];
     }
-    for (size_t b = 0; b < blk_sh.size(); ++b)
-      for (const uint4& h : blk_sh[b]) need[b] += h.z;
-    const uint64_t most = *std::max_element(need.begin(), need.end()) * sizeof(uint2);
+    const uint64_t most = *std::max_element(need.begin(), need.end()) * sizeof(uint2) +
+                          fused_heavy_bytes(a, s.persistent_blocks);
     const uint64_t bytes = std::min<uint64_t>((most + 255) & ~255ull, fused_row_smem_max());
     if (bytes >= 1024) {
       SGB_CUDA(set_fused_row_smem((uint32_t)bytes));
@@ -453,9 +482,8 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   const bool may_fuse = upd_words_n * 32u <=
                         (uint64_t)std::max(1, cfg.blocks_per_sm) * s.sm_count * kPersistBlock;
   s.ring_slots = (uint32_t)max_delay + (may_fuse ? 3u : 2u);
-  // History rows: one per delay; where the fused kernel may run with shards
-  // (delays >= 3) at least 4: in its split-barrier timeline a block may
-  // rewrite a row up to one step before a block behind it reads that row.
+  // History rows: one per delay, and at least 4 where the fused kernel may run
+  // with delays from 3 on (the layout of its checkpoints).
   s.hist_rows = (uint32_t)(may_fuse && max_delay >= 3 ? std::max(max_delay, 4) : max_delay);
   // A plastic synapse with delay d reads its pre cell's spikes d .. d +
   // window - 1 steps back, a teacher up to max_delay steps back.  Windows that
@@ -604,7 +632,7 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   size_t m = 0;
   auto take = [&](size_t bytes) { size_t o = m; m = align_up(m + std::max<size_t>(bytes, 1), 256); return o; };
   const size_t o_ctl = take(sizeof(Ctl));
-  const size_t o_bar = take(sizeof(unsigned long long));
+  const size_t o_bar = take(kBarBytes + 4 * kHeavyWords * sizeof(unsigned long long));  // and the board
   const size_t o_segs = take(nseg * sizeof(SegDev));
   const size_t o_projs = take(std::max<size_t>(s.projs.size(), 1) * sizeof(ProjDev));
   const size_t o_srcs = take(std::max<size_t>(s.srcs.size(), 1) * sizeof(SrcDev));
@@ -636,6 +664,7 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   StepArgs& a = s.args;
   a.ctl = (Ctl*)(mb + o_ctl);
   a.bar = (unsigned long long*)(mb + o_bar);
+  a.board = (unsigned long long*)(mb + o_bar + kBarBytes);
   a.segs = (const SegDev*)(mb + o_segs);
   a.projs = (const ProjDev*)(mb + o_projs);
   a.srcs = (const SrcDev*)(mb + o_srcs);
@@ -814,14 +843,6 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   if (!upd_words.empty())
     SGB_CUDA(cudaMemcpy((void*)a.upd_words, upd_words.data(), upd_words.size() * 4, cudaMemcpyHostToDevice));
   s.upd_words = upd_words;
-  if ((uint64_t)upd_words.size() * 32 <= (uint64_t)s.persistent_blocks * kPersistBlock) {
-    // Resident networks may run the fused kernel: room for its shards.
-    const size_t bytes = align_up((size_t)s.n_pad * 4, 256) +
-                         align_up((size_t)s.persistent_blocks * kMaxShards * sizeof(uint4), 256) +
-                         ((size_t)s.persistent_blocks + 1) * 4;
-    SGB_CUDA(cudaMalloc(&s.d_shard, bytes));
-    s.push_bytes += bytes;
-  }
   int rc = upload_modes(s);
   if (rc) return rc;
 
@@ -877,7 +898,7 @@ static cudaError_t issue_chunk(Sim& s, uint32_t c, cudaStream_t st, int64_t* nla
   if ((e = launch_chunk_begin(a, st))) return e;
   L++;
   if (s.cfg.exec_mode == SGB_EXEC_PERSISTENT) {
-    if ((e = cudaMemsetAsync(a.bar, 0, sizeof(unsigned long long), st))) return e;
+    if ((e = cudaMemsetAsync(a.bar, 0, kBarBytes + 4 * kHeavyWords * sizeof(unsigned long long), st))) return e;
     if ((e = launch_persistent(a, c, s.persistent_blocks, st))) return e;
     L++;
   } else {

@@ -66,10 +66,11 @@ struct Sim {
   size_t hist_bytes = 0;      // spike history + its summary
   int persistent_blocks = 0;
   std::vector<uint32_t> upd_words;  // host copy of args.upd_words
-  int64_t n_shard_cells = 0;        // cells whose delay >= 2 synapses are sharded
+  int64_t n_heavy_cells = 0;        // cells of the fused kernel's heavy words
   // Plasticity (STDP) of plastic projections.
   void* d_plast = nullptr;
-  void* d_shard = nullptr;    // fused-kernel shards: split points, shard list, per-block offsets
+  void* d_heavy = nullptr;    // fused kernel's heavy words: split points, index, lists
+  size_t heavy_bytes = 0;
   void* d_sorted = nullptr;   // dense tables in the one-barrier resident kernel's form
   size_t sorted_bytes = 0;
   size_t off_recent = 0;      // per-cell spike registers inside d_plast

@@ -20,12 +20,13 @@
 // per chunk of steps (a bounded grid barrier orders them).  The persistent
 // kernel comes in three forms: fused (every word resident in one warp, every
 // projection event-driven: update and push share one phase, one barrier a
-// step, push rows and items in shared memory; with one substep a step it
+// step, push rows in shared memory, long rows delivered by their targets'
+// blocks; with one substep a step it
 // publishes each step's spikes one step early, as soon as the potential that
 // decides them is known, and makes a step's writes after its barrier
 // arrival -- the late-push timeline, optionally with a split barrier),
-// resident (words resident,
-// some dense pulls: two barriers) and general (more words than warps; one
+// resident (words resident, some dense pulls: one barrier a step with one
+// substep, else two) and general (more words than warps; one
 // barrier a step with the pushes in each block's shared memory when every
 // projection is event-driven, else two with a global item list).  With
 // plastic projections a plasticity phase runs before the deliveries.  The
@@ -86,14 +87,16 @@ __device__ __forceinline__ bool periodic_fire(const SrcDev& s, int64_t k) {
   return floor(x1) != floor(x0);
 }
 
-__device__ bool input_fire(const StepArgs& a, const SrcDev* srcs, const SegDev& sd, uint32_t local,
-                           uint32_t mask, unsigned long long t) {
+__device__ __forceinline__ bool input_fire(const StepArgs& a, const SrcDev* srcs, const SegDev& sd,
+                                           uint32_t local, uint32_t mask, unsigned long long t) {
+  const int substeps = a.substeps;
   bool fire = false;
   U4 r{};
-  for (int s = 0; s < a.substeps; ++s) {
+#pragma unroll 1
+  for (int s = 0; s < substeps; ++s) {
     if ((s & 3) == 0) r = philox_draw(sd.seed, sd.key_base + local, t, kTagInput, (uint32_t)(s >> 2));
     const uint32_t x = u4_get(r, s & 3);
-    const int64_t k = (int64_t)t * a.substeps + s;
+    const int64_t k = (int64_t)t * substeps + s;
     uint32_t m = mask;
     while (m) {
       const int b = __ffs(m) - 1;
@@ -108,7 +111,6 @@ __device__ bool input_fire(const StepArgs& a, const SrcDev* srcs, const SegDev& 
   }
   return fire;
 }
-
 // Conductance-based LIF, `substeps` explicit Euler steps.  Statement order is
 // the reference's (Simulation_header.cu:338-370): synaptic current from the
 // old conductances, conductance decay plus the step's increment on substep 0
@@ -619,27 +621,6 @@ __device__ __forceinline__ uint32_t push_item(const StepArgs& a, uint2 it, uint3
               __float2int_rn(wv[k]));
   }
   return it.y >> 23;
-}
-
-// The same from a block's shared-memory copy of its cells' rows: {synapse
-// word, fixed-point increment} per synapse, so the item's only memory round
-// trip is its atomics.
-__device__ __forceinline__ uint32_t push_item_smem(const StepArgs& a, const uint2* rows, uint2 it,
-                                                   uint32_t slot0) {
-  constexpr int kPer = kPushChunk / 32;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t n = it.y >> 23;
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const uint32_t j = k * 32 + lane;
-    if (j >= n) break;
-    const uint2 e = rows[it.x + j];
-    uint32_t slot = slot0 + ((e.x >> kPushPostBits) & 15u);
-    if (slot >= a.ring_slots) slot -= a.ring_slots;
-    atomicAdd(a.ring + (((size_t)slot * a.n_pad + (e.x & kPushPostMask)) << 1) + (e.x >> 31),
-              (int)e.y);
-  }
-  return n;
 }
 
 // ---- dense pull (ELL) ----------------------------------------------------------
@@ -1297,13 +1278,16 @@ __host__ __device__ __forceinline__ uint32_t pull_rows(const StepArgs& a) {
 // step's entries are contiguous: its reservations all follow the previous
 // barrier).  After the launch's last barrier every count is final; block 0
 // scans them (all its threads call this; s_wsum holds kPersistBlock / 32).
-__device__ void raster_offsets_from_counts(const StepArgs& a, uint32_t n_steps, uint32_t* s_wsum) {
+__device__ __noinline__ void raster_offsets(const uint32_t* counts, uint32_t n_segs, uint32_t* raster_off,
+                                            uint32_t n_steps, uint32_t* s_wsum) {
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
   const uint32_t per = (n_steps + blockDim.x - 1) / blockDim.x;
   const uint32_t q0 = min(n_steps, threadIdx.x * per), q1 = min(n_steps, q0 + per);
   uint32_t tot = 0;
+#pragma unroll 1
   for (uint32_t q = q0; q < q1; ++q)
-    for (uint32_t g = 0; g < a.n_segs; ++g) tot += __ldcg(a.counts + (size_t)q * a.n_segs + g);
+#pragma unroll 1
+    for (uint32_t g = 0; g < n_segs; ++g) tot += __ldcg(counts + (size_t)q * n_segs + g);
   uint32_t incl = tot;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -1325,10 +1309,16 @@ __device__ void raster_offsets_from_counts(const StepArgs& a, uint32_t n_steps, 
   }
   __syncthreads();
   uint32_t run = s_wsum[wib] + incl - tot;
+#pragma unroll 1
   for (uint32_t q = q0; q < q1; ++q) {
-    for (uint32_t g = 0; g < a.n_segs; ++g) run += __ldcg(a.counts + (size_t)q * a.n_segs + g);
-    a.raster_off[q + 1] = run;
+#pragma unroll 1
+    for (uint32_t g = 0; g < n_segs; ++g) run += __ldcg(counts + (size_t)q * n_segs + g);
+    raster_off[q + 1] = run;
   }
+}
+__device__ __forceinline__ void raster_offsets_from_counts(const StepArgs& a, uint32_t n_steps,
+                                                           uint32_t* s_wsum) {
+  raster_offsets(a.counts, a.n_segs, a.raster_off, n_steps, s_wsum);
 }
 
 // General persistent kernel.  ONE (networks without dense pulls or rules that
@@ -2007,144 +1997,283 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 }
 
 // Fused form (resident networks whose projections are all event-driven): a
-// step's deliveries only target ring slots t+1 .. t+D-1 while its update only
+// step's deliveries only target ring slots t+1 .. t+D while its update only
 // reads slot t, so update and push of the same step share one phase and a
-// step needs one grid barrier.  Each block gathers the push items of its
-// spiking cells in shared memory, so the rows of a cell with thousands of
-// synapses spread over the block's 32 warps.  With a.row_smem > 0 the block
-// first copies its cells' push rows into dynamic shared memory (in word, lane
-// order, each row whole or not at all; rows past the capacity stay in global
-// memory), so a step's pushes read no global memory.
-constexpr uint32_t kBlockItems = 2048;  // push items per block and step (16 KiB)
-// Own rows are cut into items of 2^a.item_log2 synapses (32, 64 or 128; 64 =
-// two per lane unless the autotuner picked another width): a block usually
-// pushes one or two spikes' rows a step, and smaller items spread their
-// scattered reductions over more of its warps.
+// step needs one grid barrier.
+//   What bounds a step is not its mean work but its slowest block: with every
+// row pushed by the block that holds its cell, blocks did 2,900 cycles of work
+// a step on average, and the slowest of them 5,600 (a Golgi cell's 1,600
+// scattered reductions leave one SM at about three cycles each).  So long rows
+// are not pushed by their block:
+//   Heavy words (32-cell words of long rows, chosen by the host).  Every block
+// keeps the heavy cells' synapses onto its own cells in shared memory, grouped
+// by heavy cell, and an own delay line of increments (s_line) for its cells.
+// A heavy word's spikes of step t go onto a board in global memory, one 64-bit
+// word {step tag, spike bits} per heavy word; in step t one warp of every
+// block reads the board, adds what its cells receive into its line's slots t +
+// d, d >= 1, and the block barrier that ends the step hands them to the update
+// of t + 1.  Bits and tag share a word, so the board needs no fence and no
+// barrier of its own.  A Golgi spike becomes ten additions in each block's
+// shared memory.  At the end of a launch the line's pending slots are added to
+// the ring, so a launch leaves what the other kernels expect.
+//   Other rows are pushed by the spiking cell's own warp, from a copy of the
+// block's rows in shared memory (row_smem; rows past the capacity stay in
+// global memory); only rows over kDirectRow synapses, in a block that has any,
+// are cut into items for all of the block's warps, at the price of a block
+// barrier a step.
+//   A step's stimulus decisions share what does not depend on the cell: which
+// sources are on or fire periodically in each substep is worked out once per
+// block, by that warp, a lane per source and substep (s_on).
+//   Per step, start of this design -> now: 92,550 cells 2.21 -> 1.69 us, with
+// 16-bit weights 2.46 -> 1.73; 9,256 cells 1.70 -> 1.48; 152,700 cells (two words
+// a warp) 2.71 -> 2.08; 92,550 cells in steps of ten substeps 6.6 -> 4.4.
+constexpr uint32_t kBlockItems = 1024;  // push items per block and step (8 KiB)
+constexpr uint32_t kDirectRow = 256;    // longest row that its cell's warp pushes by itself
+constexpr uint32_t kSrcCache = 16;      // stimulus sources kept in shared memory
+constexpr uint32_t kOnSubsteps = 32;    // substeps whose source states are shared
+// Items are ranges of 2^a.item_log2 synapses (64 or 128) of a long row: (first
+// synapse, length << 23 | 1 when it is in shared memory).
+// States of n_srcs sources in the substeps of step t, by the lanes of one warp.
+__device__ __forceinline__ void source_states(const SrcDev* srcs, uint2* on, uint32_t n_srcs,
+                                           uint32_t substeps, unsigned long long t) {
+  const uint32_t lane = threadIdx.x & 31u;
+  if (lane < substeps) on[lane] = make_uint2(0u, 0u);
+  __syncwarp();
+#pragma unroll 1
+  for (uint32_t p = lane; p < n_srcs * substeps; p += 32u) {
+    const uint32_t s = p / n_srcs, j = p - s * n_srcs;
+    const SrcDev& src = srcs[j];
+    const int64_t k = (int64_t)t * substeps + s;
+    if (!window_on(src, k)) continue;
+    if (src.kind == SGB_INPUT_POISSON)
+      atomicOr(&on[s].x, 1u << j);
+    else if (periodic_fire(src, k))
+      atomicOr(&on[s].y, 1u << j);
+  }
+  __syncwarp();
+}
 
-// An item of the fused kernel: (first synapse, length << 23 | flags); flag 1:
-// the synapses are in the block's shared-memory rows, flag 2: a shard of the
-// previous step's spike (its delays count from that step's ring slot).
-template <bool BF16>
-__device__ __forceinline__ uint32_t push_any(const StepArgs& a, const uint2* rows, uint2 it,
-                                             uint32_t slot, uint32_t prev) {
-  const uint32_t s0 = (it.y & 2u) ? prev : slot;
-  return (it.y & 1u) ? push_item_smem(a, rows, it, s0) : push_item<BF16>(a, it, s0);
+// Shared memory of the heavy words: the line, where each heavy cell's synapses
+// start, and up to hv_cap of them.
+__host__ __device__ __forceinline__ uint32_t hv_line_slots(const StepArgs& a) { return a.max_delay + 1u; }
+__host__ __device__ __forceinline__ size_t hv_bytes(const StepArgs& a, uint32_t blocks) {
+  if (!a.hv_words) return 0;
+  const size_t cells = ((size_t)a.n_upd_words + blocks - 1u) / blocks * 32u;
+  const size_t line = hv_line_slots(a) * cells * sizeof(int2);
+  const size_t off = ((size_t)(a.hv_words * 32u + 1u) * sizeof(uint16_t) + 15) & ~(size_t)15;
+  return line + off + (size_t)a.hv_cap * sizeof(uint2);
+}
+
+// Words of a block, at most: one per warp up to kFusedSingle, else two.
+constexpr uint32_t kFusedSingle = 22;  // beyond, 24 warps of 80 registers are not enough
+__host__ __device__ constexpr uint32_t fused_max_words(uint32_t w) {
+  return w == 1u ? kFusedSingle : (uint32_t)kPersistBlock / 32u;
+}
+__host__ __device__ constexpr uint32_t fused_max_threads(uint32_t w) {
+  return 32u * ((fused_max_words(w) + w - 1u) / w + 2u);
 }
 
 // TL: the step's timeline -- 0 spikes in their own step; for one-substep steps
 // 1 late push, 2 late push with a split grid barrier (see the loops below).
-// ILOG: push items of 2^ILOG synapses.
-template <bool BF16, uint32_t TL, uint32_t ILOG>
-__global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_fused(StepArgs a,
-                                                                       uint32_t n_steps) {
+// W: words per warp.  A warp that holds two words shares a step's bookkeeping
+// between them and has two independent chains of loads and arithmetic in
+// flight, and the smaller block has the registers for it (with the shared
+// memory this kernel takes, little is left for L1, and a spilled register
+// costs an L2 round trip).  Two more warps hold no word: the last keeps the grid
+// barrier, the one before it reads the board and prepares the sources.
+template <bool BF16, uint32_t TL, uint32_t W>
+__global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(StepArgs a,
+                                                                              uint32_t n_steps) {
   __shared__ uint2 s_items[kBlockItems];
   __shared__ uint32_t s_n[2];  // item count of step parity p; the other one is reset
   __shared__ uint32_t s_wsum[kPersistBlock / 32];
-  __shared__ uint4 s_sh[kMaxShards];  // {cell, first synapse, length << 23 | flags, global first}
-  __shared__ uint32_t s_shtot, s_ptot;
-  __shared__ uint32_t s_od[kPersistBlock];  // out-degree of each thread's cell
+  __shared__ uint32_t s_ptot;
+  // Out-degree of each of the block's cells (word j of the block: cells 32 j ..).
+  __shared__ uint32_t s_od[fused_max_words(W) * 32u];
   // Segment descriptors and stimulus sources, read every step, in shared
   // memory (when few enough): a miss in the small L1 that this kernel's
   // shared-memory carve-out leaves would cost an L2 round trip per step.
-  constexpr uint32_t kSegCache = 16, kSrcCache = 16;
+  constexpr uint32_t kSegCache = 16;
   __shared__ SegDev s_seg[kSegCache];
   __shared__ SrcDev s_src[kSrcCache];
-  extern __shared__ uint2 s_rows[];
+  // Sources by substep of step t, buffer t mod 2: Poisson sources that are on,
+  // periodic sources that fire.
+  __shared__ uint2 s_on[2][kOnSubsteps];
+  __shared__ int s_ok[2], s_board_ok;
+  extern __shared__ uint2 s_dyn[];
+  const uint32_t n_thr = blockDim.x, n_wrp = n_thr >> 5, last = n_wrp - 1u;  // fused_threads
+  const uint32_t aide = last - 1u, nw = aide;  // nw: warps that may hold words
+  const bool heavy = a.hv_words != 0u && gridDim.x == a.hv_grid;
+  const uint32_t n_own = (a.n_upd_words + gridDim.x - 1u) / gridDim.x;  // words of a block, at most
+  const uint32_t nwk = (n_own + W - 1u) / W;                            // warps that hold them
+  const uint32_t n_line = hv_line_slots(a), n_cell = n_own * 32u;
+  int2* s_line = reinterpret_cast<int2*>(s_dyn);  // [n_line][n_cell]
+  uint16_t* s_hoff = reinterpret_cast<uint16_t*>(s_line + (heavy ? n_line * n_cell : 0u));
+  uint2* s_rows = s_dyn + hv_bytes(a, gridDim.x) / sizeof(uint2);
+  uint2* s_hsyn = s_rows - (heavy ? a.hv_cap : 0u);
   const SegDev* segs = a.n_segs <= kSegCache ? s_seg : a.segs;
   const SrcDev* srcs = a.n_srcs <= kSrcCache ? s_src : a.srcs;
+  const bool shared_src = a.n_srcs <= kSrcCache && a.substeps <= (int)kOnSubsteps;
   if (a.n_segs <= kSegCache && threadIdx.x < a.n_segs) s_seg[threadIdx.x] = a.segs[threadIdx.x];
   if (a.n_srcs <= kSrcCache && threadIdx.x < a.n_srcs) s_src[threadIdx.x] = a.srcs[threadIdx.x];
   Ctl* ctl = a.ctl;
-  StepIdx ix = step_of(a);
-  const unsigned long long t0 = ix.t;
+  const StepIdx ix0 = step_of(a);
+  const unsigned long long t0 = ix0.t;
+  uint32_t slot = ix0.slot;  // ring slot of the step at hand
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t wib = threadIdx.x >> 5;
   const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
-  // Words are dealt round-robin over the blocks (word slot = warp x blocks +
-  // block), so every SM holds about the same number of cells and spikes.
-  const uint32_t ws = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const bool has = ws < a.n_upd_words;
+  // Words are dealt round-robin over the blocks (word j of block b is slot j x
+  // blocks + b), so every SM holds about the same number of cells and spikes;
+  // warp v holds the block's words v and v + nwk.
   // st: a LIF cell's state {u, g0, g1, ref}; an input cell's source mask and
   // index within its segment (bits of st.x, st.y).
-  uint32_t w = 0, seg = 0, i = 0, r0 = 0, r1 = 0;
-  s_od[threadIdx.x] = 0;
-  bool valid = false, lif = false;
-  float4 st = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (has) {
-    w = __ldg(a.upd_words + ws);
-    seg = __ldg(a.seg_of_word + w);
-    i = (w << 5) + lane;
-    const SegDev& sd = a.segs[seg];
-    const uint32_t local = i - sd.base;
-    valid = local < sd.count;
-    lif = sd.kind == kSegLif;
-    if (valid) {
-      if (lif)
-        st = state_in(a.su[i], a.sg[i], sd.Vr);
-      else
-        st = make_float4(__uint_as_float(__ldg(a.src_mask + i)), __uint_as_float(local), 0.f, 0.f);
-      s_od[threadIdx.x] = __ldg(a.outdeg + i);
-      r0 = __ldg(a.push_row + i);
-      r1 = __ldg(a.push_row + i + 1);
-    }
-  }
-  // Shards: a sharded cell pushes only its delay-1 and delay-2 synapses (r1
-  // becomes its split point); the rest of its row is cut into shards dealt to
-  // blocks, which push a shard in the step after the cell's spike (two steps
-  // after it in the late-push timeline), reading the spike from the history.
-  // Its delays d >= 3 count from the spike's ring slot, so the targets are
-  // still ahead of the updates that read them.
-  // This block's n_sh shards go first into shared memory while they fit.
-  const bool sharded = a.n_shards != 0 && gridDim.x == a.shard_grid;
-  uint32_t n_sh = 0;
-  if (sharded) {
-    if (valid) r1 = __ldg(a.push_split + i);
-    const uint32_t h0 = __ldg(a.shard_off + blockIdx.x);
-    n_sh = __ldg(a.shard_off + blockIdx.x + 1) - h0;
-    if (threadIdx.x == 0) {
-      const uint32_t cap = a.row_smem / (uint32_t)sizeof(uint2);
-      uint32_t used = 0;
-      for (uint32_t j = 0; j < n_sh; ++j) {
-        const uint4 h = a.shards[h0 + j];
-        const bool in = h.z <= cap - used;
-        s_sh[j] = make_uint4(h.x, in ? used : h.y, (h.z << 23) | (in ? 3u : 2u), h.y);
-        if (in) used += h.z;
+  bool has[W], valid[W], lif[W], rd[W];
+  uint32_t seg[W], i[W], cell[W], hw[W];  // cell: index in the block
+  uint2 row[W];                           // first synapse, length | 1 << 31 when in shared memory
+  float4 st[W];
+#pragma unroll
+  for (uint32_t k = 0; k < W; ++k) {
+    const uint32_t j = wib + k * nwk, ws = j * gridDim.x + blockIdx.x;
+    has[k] = wib < nwk && j < n_own && ws < a.n_upd_words;
+    valid[k] = lif[k] = false;
+    seg[k] = i[k] = 0;
+    hw[k] = 0xFFFFu;
+    cell[k] = has[k] ? j * 32u + lane : 0u;
+    st[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    row[k] = make_uint2(0u, 0u);
+    if (has[k]) {
+      const uint32_t w = __ldg(a.upd_words + ws);
+      seg[k] = __ldg(a.seg_of_word + w);
+      i[k] = (w << 5) + lane;
+      const SegDev& sd = a.segs[seg[k]];
+      const uint32_t local = i[k] - sd.base;
+      valid[k] = local < sd.count;
+      lif[k] = sd.kind == kSegLif;
+      if (heavy) hw[k] = __ldg(a.hv_index + w);
+      uint32_t od = 0;
+      if (valid[k]) {
+        if (lif[k])
+          st[k] = state_in(a.su[i[k]], a.sg[i[k]], sd.Vr);
+        else
+          st[k] = make_float4(__uint_as_float(__ldg(a.src_mask + i[k])), __uint_as_float(local), 0.f, 0.f);
+        od = __ldg(a.outdeg + i[k]);
+        const uint32_t r0 = __ldg(a.push_row + i[k]);
+        const uint32_t r1 = heavy ? __ldg(a.push_split + i[k]) : __ldg(a.push_row + i[k] + 1);
+        row[k] = make_uint2(r0, r1 - r0);
       }
-      s_shtot = used;
+      s_od[cell[k]] = od;
     }
-    __syncthreads();
-    for (uint32_t j = wib; j < n_sh; j += kPersistBlock / 32) {
-      const uint4 h = s_sh[j];
-      if (h.z & 1u)
-        for (uint32_t k = lane; k < (h.z >> 23); k += 32)
-          s_rows[h.y + k] = make_uint2(__ldg(a.push_syn + h.w + k),
-                                       (uint32_t)__float2int_rn(load_weight<BF16>(a.push_w, h.w + k)));
-    }
+    rd[k] = lif[k] && valid[k];
   }
-  // Input cells: the stimulus decision of the coming step, drawn ahead (it
-  // depends only on the step index) -- for later steps while the previous
-  // grid barrier completes.
-  const bool stim = valid && !lif && __float_as_uint(st.x) != 0u;
-  // The barrier is polled from the highest warp without stimulated cells, so
-  // the poll starts as soon as the block has arrived.
-  __shared__ uint32_t s_poller;
-  if (threadIdx.x == 0) s_poller = 0;
-  __syncthreads();  // also publishes s_seg / s_src
-  bool next_in = stim && input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), t0);
-  const bool warp_stim = __any_sync(kFull, stim);
-  if (lane == 0 && !warp_stim) atomicMax(&s_poller, threadIdx.x);
-  // Push rows into shared memory: sb = the row's offset there, or kNoRow.
-  // Rows of at least kLongRow synapses are placed first (a spike of such a
-  // cell is the most work to push), then the others, each in word order.
-  constexpr uint32_t kNoRow = 0xFFFFFFFFu;
+  if (heavy) {
+    for (uint32_t j = threadIdx.x; j < n_line * n_cell; j += n_thr) s_line[j] = make_int2(0, 0);
+    const uint32_t n_off = a.hv_words * 32u + 1u;
+    const uint16_t* off = a.hv_off + (size_t)blockIdx.x * n_off;
+    for (uint32_t j = threadIdx.x; j < n_off; j += n_thr) s_hoff[j] = __ldg(off + j);
+    const uint32_t n = __ldg(off + n_off - 1u);
+    const uint2* src = a.hv_syn + (size_t)blockIdx.x * a.hv_cap;
+    for (uint32_t j = threadIdx.x; j < n; j += n_thr) s_hsyn[j] = __ldg(src + j);
+  }
+  uint32_t stim = 0;  // bit k: the thread's cell of word k is a stimulated input cell
+#pragma unroll
+  for (uint32_t k = 0; k < W; ++k)
+    if (valid[k] && !lif[k] && __float_as_uint(st[k].x) != 0u) stim |= 1u << k;
+  if (threadIdx.x == 0) {
+    s_n[0] = s_n[1] = 0;
+    s_board_ok = 1;
+  }
+  const bool blk_stim = __syncthreads_or((int)stim) != 0;  // also publishes s_seg / s_src
+  auto sources = [&](unsigned long long t) {
+    source_states(s_src, s_on[t & 1ull], a.n_srcs, (uint32_t)a.substeps, t);
+  };
+  // Element k of a pair, without indexing registers.
+  auto pick = [](uint32_t k, uint32_t x, uint32_t y) { return k ? y : x; };
+  // The stimulus decisions of the thread's input cells in step t, bit k for word k.
+  auto draw = [&](unsigned long long t) -> uint32_t {
+    uint32_t fire = 0;
+#pragma unroll 1
+    for (uint32_t k = 0; k < W; ++k) {
+      if (!((stim >> k) & 1u)) continue;
+      const SegDev& sd = segs[pick(k, seg[0], seg[W - 1])];
+      const uint32_t mask = __float_as_uint(k ? st[W - 1].x : st[0].x);
+      const uint32_t local = __float_as_uint(k ? st[W - 1].y : st[0].y);
+      if (!shared_src) {
+        fire |= (input_fire(a, srcs, sd, local, mask, t) ? 1u : 0u) << k;
+        continue;
+      }
+      bool f = false;
+      U4 r{};
+#pragma unroll 1
+      for (int s = 0; s < a.substeps; ++s) {
+        if ((s & 3) == 0) r = philox_draw(sd.seed, sd.key_base + local, t, kTagInput, (uint32_t)(s >> 2));
+        const uint32_t x = u4_get(r, s & 3);
+        const uint2 on = s_on[t & 1ull][s];
+        f |= (mask & on.y) != 0u;
+#pragma unroll 1
+        for (uint32_t m = mask & on.x; m; m &= m - 1u) f |= (uint64_t)x < s_src[__ffs(m) - 1].thresh;
+      }
+      fire |= (f ? 1u : 0u) << k;
+    }
+    return fire;
+  };
+  const bool shared_on = blk_stim && shared_src;
+  uint32_t walked = 0;
+  constexpr uint32_t kBatch = W == 1u ? 2u : 3u;  // synapses a lane has in flight; one more would spill
+  // Pushes m synapses from b0 of the block's rows or of the table; delays count
+  // from ring slot `own`.
+  auto push_range = [&](uint32_t b0, uint32_t m, bool smem, uint32_t own) {
+#pragma unroll 1
+    for (uint32_t j0 = lane; j0 < m; j0 += 32u * kBatch) {
+      uint2 e[kBatch];
+#pragma unroll
+      for (uint32_t k = 0; k < kBatch; ++k) {
+        const uint32_t j = j0 + 32u * k;
+        if (j >= m) break;
+        e[k] = smem ? s_rows[b0 + j]
+                    : make_uint2(__ldg(a.push_syn + b0 + j),
+                                 (uint32_t)__float2int_rn(load_weight<BF16>(a.push_w, b0 + j)));
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kBatch; ++k) {
+        if (j0 + 32u * k >= m) break;
+        uint32_t slot = own + ((e[k].x >> kPushPostBits) & 15u);
+        if (slot >= a.ring_slots) slot -= a.ring_slots;
+        atomicAdd(a.ring + (((size_t)slot * a.n_pad + (e[k].x & kPushPostMask)) << 1) + (e[k].x >> 31),
+                  (int)e[k].y);
+      }
+    }
+    walked += m;
+  };
+  // Input cells: the decision of the coming step is drawn ahead (it depends
+  // only on the step index).  The launch's first two come from the general
+  // form; the loops draw the later ones with the shared source states.
+  uint32_t next_in = 0, next1 = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < W; ++k)
+    if ((stim >> k) & 1u) {
+#pragma unroll 1
+      for (uint32_t q = 0; q < 2u && q < n_steps; ++q) {
+        const bool f = input_fire(a, srcs, segs[seg[k]], __float_as_uint(st[k].y), __float_as_uint(st[k].x), t0 + q);
+        if (f) (q ? next1 : next_in) |= 1u << k;
+      }
+      if (shared_src) st[k].x = __uint_as_float(__float_as_uint(st[k].x) << segs[seg[k]].src_first);
+    }
+  // Push rows into shared memory.  Rows of at least kLongRow synapses are
+  // placed first (a spike of such a cell is the most work to push), then the
+  // others, each in word order; a row that no longer fits stays in global memory.
   constexpr uint32_t kLongRow = 128;
-  uint32_t sb = kNoRow;
-  const uint32_t len = r1 - r0;
-  if (a.row_smem) {
-    const uint32_t cap = a.row_smem / (uint32_t)sizeof(uint2);
-    uint32_t used = sharded ? s_shtot : 0u;
-    for (uint32_t pass = 0; pass < 2; ++pass) {
-      const uint32_t lp = (len >= kLongRow) == (pass == 0) ? len : 0u;
+  const size_t hv = hv_bytes(a, gridDim.x);
+  const uint32_t cap = a.row_smem > hv ? (uint32_t)((a.row_smem - hv) / sizeof(uint2)) : 0u;
+  uint32_t used = 0;
+  bool has_long = false;
+#pragma unroll
+  for (uint32_t k = 0; k < W; ++k) has_long |= row[k].y > kDirectRow;
+#pragma unroll 1
+  for (uint32_t pass = 0; pass < 2u && cap; ++pass) {
+#pragma unroll
+    for (uint32_t k = 0; k < W; ++k) {
+      const uint32_t lp = !(row[k].y >> 31) && (row[k].y >= kLongRow) == (pass == 0) ? row[k].y : 0u;
       uint32_t incl = lp;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -2155,7 +2284,7 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_fused(StepArgs 
       if (lane == 31) s_wsum[wib] = incl;
       __syncthreads();
       if (wib == 0) {
-        uint32_t x = s_wsum[lane], xi = x;
+        uint32_t x = lane < n_wrp ? s_wsum[lane] : 0u, xi = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const uint32_t v = __shfl_up_sync(kFull, xi, o);
@@ -2166,384 +2295,374 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent_fused(StepArgs 
       }
       __syncthreads();
       const uint32_t base = used + s_wsum[wib] + incl - lp;
-      if (lp && base <= cap && lp <= cap - base) sb = base;
       used += s_ptot;
-    }
-    uint32_t todo = __ballot_sync(kFull, sb != kNoRow);
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const uint32_t q0 = __shfl_sync(kFull, r0, src), n = __shfl_sync(kFull, len, src);
-      const uint32_t b0 = __shfl_sync(kFull, sb, src);
-      for (uint32_t k = lane; k < n; k += 32)
-        s_rows[b0 + k] = make_uint2(__ldg(a.push_syn + q0 + k),
-                                    (uint32_t)__float2int_rn(load_weight<BF16>(a.push_w, q0 + k)));
+      const bool fits = lp && base <= cap && lp <= cap - base;
+      uint32_t todo = __ballot_sync(kFull, fits);
+#pragma unroll 1
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t q0 = __shfl_sync(kFull, row[k].x, src), n = __shfl_sync(kFull, lp, src);
+        const uint32_t b0 = __shfl_sync(kFull, base, src);
+        for (uint32_t j = lane; j < n; j += 32)
+          s_rows[b0 + j] = make_uint2(__ldg(a.push_syn + q0 + j),
+                                      (uint32_t)__float2int_rn(load_weight<BF16>(a.push_w, q0 + j)));
+      }
+      if (fits) row[k] = make_uint2(base, lp | 0x80000000u);
     }
   }
-  // From here a row is (qb, rl): its first synapse in shared or global
-  // memory and its length, with bit 31 set when it is in shared memory.
-  const uint32_t qb = sb != kNoRow ? sb : r0;
-  const uint32_t rl = len | (sb != kNoRow ? 0x80000000u : 0u);
-  constexpr uint32_t clog = ILOG, chunk = 1u << ILOG;  // push-item width
+  const bool blk_long = __syncthreads_or((int)has_long) != 0;  // also: rows are in place
+  const uint32_t clog = a.item_log2, chunk = 1u << clog;  // push-item width
   unsigned long long target = 0;
-  uint32_t walked = 0;
   bool aborted = false;
-  if (threadIdx.x == 0) s_n[0] = s_n[1] = 0;
-  __syncthreads();
-  // off / nit: the lane's first item in the block's list and its item count
-  // (a warp delivers its own items past the list's capacity).
-  uint32_t off = 0, nit = 0;
-  // Spike bookkeeping of this warp's word for the spikes of step px.t (chunk
-  // row `rel`): history and summary bits, per-segment count, events, raster
-  // entries, and the spiking cells' rows cut into chunk-synapse items
-  // in the block's list of parity `par`.
-  auto publish = [&](bool fired, const StepIdx& px, uint32_t rel, uint32_t par) {
-    off = 0;
-    nit = 0;
-    const uint32_t ballot = __ballot_sync(kFull, fired);
-    if (lane == 0) put_hist(a, px, w, ballot);
-    if (!ballot) return;
-    const uint32_t n = __popc(ballot);
-    const uint32_t rank = __popc(ballot & ((1u << lane) - 1u));
-    const uint32_t ev = __reduce_add_sync(kFull, fired ? s_od[threadIdx.x] : 0u);
-    nit = fired ? ((rl & 0x7FFFFFFFu) + chunk - 1) >> clog : 0u;
-    uint32_t incl = nit;
+  // History and summary rows are for the other kernels and the host: a launch
+  // writes those of its last hist_rows steps (rel: chunk step), and clears their
+  // summary rows and its successor's before.
+  const uint32_t n_hist = a.hist_rows;
+  auto keeps = [&](uint32_t rel) { return rel + n_hist >= n_steps; };
+  auto clear_summary = [&](uint32_t rel, uint32_t gtid, uint32_t gthreads) {
+    if (!keeps(rel) || rel > n_steps) return;
+    const uint32_t row = (ix0.srow + rel) % (n_hist + 1u);
+    for (uint32_t j = gtid; j < a.n_swords; j += gthreads)
+      __stcg(a.hsum + (size_t)row * a.n_swords + j, 0u);
+  };
+  // Spike bookkeeping of this warp's words for the spikes of chunk step `rel`
+  // (ring slot px; fired: bit k for word k): the board, history, per-segment
+  // count, events, raster entries; then the spiking cells' rows, pushed from
+  // here, or cut into the items of parity rel & 1.
+  auto publish = [&](uint32_t fired, uint32_t rel, uint32_t px) {
+    uint32_t b[W];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(kFull, incl, o);
-      if (lane >= (uint32_t)o) incl += v;
+    for (uint32_t k = 0; k < W; ++k) b[k] = __ballot_sync(kFull, (fired >> k) & 1u);
+    if ((hw[0] & hw[W - 1]) != 0xFFFFu && lane < W) {
+      const uint32_t h = pick(lane, hw[0], hw[W - 1]);
+      const unsigned long long v = ((unsigned long long)(rel + 1u) << 32) | pick(lane, b[0], b[W - 1]);
+      if (h != 0xFFFFu)
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(a.board + (rel & 3u) * kHeavyWords + h),
+                     "l"(v) : "memory");
     }
-    const uint32_t tot = __shfl_sync(kFull, incl, 31);
-    uint32_t roff = 0;
-    if (lane == 0) {
-      if (tot) off = atomicAdd(&s_n[par], tot);
-      atomicAdd(&a.counts[(size_t)rel * a.n_segs + seg], n);
-      if (ev) atomicAdd(&ctl->events, (unsigned long long)ev);
-      if (a.raster_cap) roff = atomicAdd(&ctl->raster_count, n);
+    if (keeps(rel) && lane == 0) {
+      StepIdx hx = ix0;
+      hx.hrow = (ix0.hrow + rel) % n_hist;
+      hx.srow = (ix0.srow + rel) % (n_hist + 1u);
+      ix_rows(a, hx);
+#pragma unroll
+      for (uint32_t k = 0; k < W; ++k)
+        if (has[k]) put_hist(a, hx, i[k] >> 5, b[k]);
     }
-    off = __shfl_sync(kFull, off, 0) + incl - nit;
-    for (uint32_t k = 0; k < nit && off + k < kBlockItems; ++k) {
-      const uint32_t q = k << clog;
-      s_items[off + k] = make_uint2(qb + q, (min(chunk, (rl & 0x7FFFFFFFu) - q) << 23) |
-                                                (rl >> 31));
-    }
-    if (a.raster_cap) {
-      roff = __shfl_sync(kFull, roff, 0);
-      if (fired) {
-        if (roff + rank < a.raster_cap)
-          a.raster[roff + rank] = raster_record(i, rel);
-        else
-          atomicOr(&ctl->error, kErrRasterOverflow);
+    if (__builtin_expect((b[0] | b[W - 1]) == 0u, 0)) return;
+#pragma unroll 1
+    for (uint32_t k = 0; k < W; ++k) {
+      const uint32_t ballot = pick(k, b[0], b[W - 1]);
+      if (!ballot) continue;
+      const bool mine = (ballot >> lane) & 1u;
+      if (lane == 0)
+        atomicAdd(&a.counts[(size_t)rel * a.n_segs + pick(k, seg[0], seg[W - 1])], (uint32_t)__popc(ballot));
+      if (mine) atomicAdd(&ctl->events, (unsigned long long)s_od[pick(k, cell[0], cell[W - 1])]);
+      const uint32_t rx = pick(k, row[0].x, row[W - 1].x), ry = pick(k, row[0].y, row[W - 1].y);
+      const uint32_t n = ry & 0x7FFFFFFFu;
+      uint32_t todo = __ballot_sync(kFull, mine && n != 0u && n <= kDirectRow);
+#pragma unroll 1
+      while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const uint32_t b0 = __shfl_sync(kFull, rx, src), l0 = __shfl_sync(kFull, ry, src);
+        push_range(b0, l0 & 0x7FFFFFFFu, (l0 >> 31) != 0u, px);
+      }
+      if (blk_long) {
+        // Long rows: items of the block's list, and from here what it has no room for.
+        uint32_t from = 0;
+        const bool is_long = mine && n > kDirectRow;
+        if (is_long) {
+          const uint32_t nit = (n + chunk - 1u) >> clog;
+          const uint32_t off = atomicAdd(&s_n[rel & 1u], nit);
+          const uint32_t put = off < kBlockItems ? min(nit, kBlockItems - off) : 0u;
+#pragma unroll 1
+          for (uint32_t q = 0; q < put; ++q)
+            s_items[off + q] = make_uint2(rx + (q << clog), (min(chunk, n - (q << clog)) << 23) | (ry >> 31));
+          from = min(n, put << clog);
+        }
+        todo = __ballot_sync(kFull, is_long && from < n);
+#pragma unroll 1
+        while (todo) {
+          const int src = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          const uint32_t b0 = __shfl_sync(kFull, rx, src), l0 = __shfl_sync(kFull, ry, src);
+          const uint32_t f0 = __shfl_sync(kFull, from, src);
+          push_range(b0 + f0, (l0 & 0x7FFFFFFFu) - f0, (l0 >> 31) != 0u, px);
+        }
+      }
+      if (a.raster_cap) {
+        uint32_t roff = 0;
+        if (lane == 0) roff = atomicAdd(&ctl->raster_count, (uint32_t)__popc(ballot));
+        roff = __shfl_sync(kFull, roff, 0);
+        if (mine) {
+          const uint32_t to = roff + __popc(ballot & ((1u << lane) - 1u));
+          if (to < a.raster_cap)
+            a.raster[to] = raster_record(pick(k, i[0], i[W - 1]), rel);
+          else
+            atomicOr(&ctl->error, kErrRasterOverflow);
+        }
       }
     }
   };
-  // A spiking shard (its cell's bit set in the history word sh_w) becomes
-  // chunk-synapse items of parity par; returns the first item past the
-  // list's capacity, which this thread's warp pushes itself (kNoRow: none).
-  auto shard_items = [&](bool ck, uint32_t sh_w, uint32_t par) -> uint32_t {
-    uint32_t from = kNoRow;
-    if (ck) {
-      const uint4 h = s_sh[threadIdx.x];
-      if ((sh_w >> (h.x & 31u)) & 1u) {
-        const uint32_t sl = h.z >> 23, ni = (sl + chunk - 1) >> clog;
-        const uint32_t o = atomicAdd(&s_n[par], ni);
-        for (uint32_t k = 0; k < ni && o + k < kBlockItems; ++k)
-          s_items[o + k] = make_uint2(h.y + (k << clog),
-                                      (min(chunk, sl - (k << clog)) << 23) | (h.z & 3u));
-        if (o + ni > kBlockItems) from = o < kBlockItems ? kBlockItems - o : 0u;
-      }
-    }
-    return from;
-  };
-  // The block's items of parity par, then the items past the list's
-  // capacity; own rows count their delays from ring slot `own`, shards from
-  // ring slot `shard` (their spike's step).
-  // nw: the warps that deliver (the first nw of the block; fewer than all of
-  // them meet on block barrier 1 instead of 0).
-  auto deliver = [&](uint32_t par, uint32_t own, uint32_t shard, uint32_t sh_from,
-                     uint32_t nw = kPersistBlock / 32) {
-    if (nw == kPersistBlock / 32) __syncthreads(); else bar_sync_first(nw * 32u);
+  // Blocks with long rows: the items of parity par, by the first n_w warps (when
+  // not all, they meet on block barrier 1); delays count from ring slot `own`.
+  auto deliver = [&](uint32_t par, uint32_t own, uint32_t n_w) {
+    if (!blk_long) return;
+    if (n_w == n_wrp) __syncthreads(); else bar_sync_first(n_w * 32u);
     const uint32_t n_items = min(s_n[par], kBlockItems);
     // The other parity's count was last read before this block barrier.
     if (threadIdx.x == 0) s_n[par ^ 1u] = 0;
-    for (uint32_t u = wib; u < n_items; u += nw)
-      walked += push_any<BF16>(a, s_rows, s_items[u], own, shard);
-    uint32_t spill = __ballot_sync(kFull, off + nit > kBlockItems);
-    while (spill) {
-      const int src = __ffs(spill) - 1;
-      spill &= spill - 1;
-      const uint32_t o = __shfl_sync(kFull, off, src), c = __shfl_sync(kFull, nit, src);
-      const uint32_t b0 = __shfl_sync(kFull, qb, src), bl = __shfl_sync(kFull, rl, src);
-      for (uint32_t k = o < kBlockItems ? kBlockItems - o : 0; k < c; ++k) {
-        const uint32_t q = k << clog;
-        const uint2 it = make_uint2(b0 + q, (min(chunk, (bl & 0x7FFFFFFFu) - q) << 23) | (bl >> 31));
-        walked += push_any<BF16>(a, s_rows, it, own, shard);
+#pragma unroll 1
+    for (uint32_t u = wib; u < n_items; u += n_w) {
+      const uint2 it = s_items[u];
+      push_range(it.x, it.y >> 23, (it.y & 1u) != 0u, own);
+    }
+  };
+  // The heavy words' spikes of chunk step rel into the line, whose slot of that
+  // step is `at`; one warp.  A word's tag comes before its owner's arrival
+  // at the barrier that this step waits for; the wait has that barrier's limit.
+  auto board = [&](uint32_t rel, uint32_t at) {
+    // Up to four words per lane, read together.
+    uint32_t got[kHeavyWords / 32u];
+    {
+      const unsigned long long* p = a.board + (rel & 3u) * kHeavyWords + lane;
+      unsigned long long w0 = 0;
+      uint32_t it = 0;
+      while (true) {
+        bool all = true;
+        unsigned long long v[kHeavyWords / 32u];
+#pragma unroll
+        for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) {
+          v[k] = (unsigned long long)(rel + 1u) << 32;
+          if (lane + 32u * k < a.hv_words)
+            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v[k]) : "l"(p + 32u * k) : "memory");
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) {
+          all = all && (uint32_t)(v[k] >> 32) == rel + 1u;
+          got[k] = (uint32_t)v[k];
+        }
+        if (__all_sync(kFull, all)) break;
+        if ((++it & 255u) == 0u) {
+          const unsigned long long now = global_ns();
+          if (w0 == 0) w0 = now;
+          const bool out = now - w0 > kBarrierTimeoutNs || (__ldcg(&ctl->error) & kErrBarrierTimeout);
+          if (__any_sync(kFull, out)) {
+            if (lane == 0) {
+              atomicOr(&ctl->error, kErrBarrierTimeout);
+              s_board_ok = 0;
+            }
+            return;
+          }
+        }
+        __nanosleep(32);
       }
     }
-    if (n_sh) {
-      uint32_t sp = __ballot_sync(kFull, sh_from != kNoRow);
-      while (sp) {
-        const int src = __ffs(sp) - 1;
-        sp &= sp - 1;
-        const uint4 h = s_sh[wib * 32u + src];
-        const uint32_t sl = h.z >> 23;
-        for (uint32_t q = __shfl_sync(kFull, sh_from, src) << clog; q < sl; q += chunk)
-          walked += push_any<BF16>(
-              a, s_rows, make_uint2(h.y + q, (min(chunk, sl - q) << 23) | (h.z & 3u)), own,
-              shard);
+#pragma unroll
+    for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) {
+      const uint32_t k0 = 32u * k, bits = got[k];
+      uint32_t words = __ballot_sync(kFull, bits != 0u);
+#pragma unroll 1
+      while (words) {
+        const int src = __ffs(words) - 1;
+        words &= words - 1u;
+        uint32_t b = __shfl_sync(kFull, bits, src);
+#pragma unroll 1
+        while (b) {
+          const uint32_t c = (k0 + src) * 32u + __ffs(b) - 1u;
+          b &= b - 1u;
+          const uint32_t q1 = s_hoff[c + 1u];
+          walked += q1 - s_hoff[c];
+#pragma unroll 1
+          for (uint32_t q = s_hoff[c] + lane; q < q1; q += 32u) {
+            const uint2 e = s_hsyn[q];  // {cell | delay << 10 | accumulator << 14, increment}
+            uint32_t slot = at + ((e.x >> 10) & 15u);
+            if (slot >= n_line) slot -= n_line;
+            atomicAdd(reinterpret_cast<int*>(s_line + slot * n_cell + (e.x & 1023u)) + (e.x >> 14), (int)e.y);
+          }
+        }
       }
     }
   };
-  // The shards of the spikes of step ix.t - 1 (ix has advanced past that
-  // step): the epilogue of the timelines that push shards a step late.
-  auto last_shards = [&]() {
-    const uint32_t prev = ix.slot == 0u ? a.ring_slots - 1u : ix.slot - 1u;
-    bool hit = false;
-    if (threadIdx.x < n_sh) {
-      const uint32_t c = s_sh[threadIdx.x].x;
-      hit = (__ldcg(hist_base(a, ix.hrow) + a.n_words + (c >> 5)) >> (c & 31u)) & 1u;
+  // The increments of the thread's cells in ring slot `slot` and the line's slot
+  // `at`; clear_in takes them out of the ring (the line's go as they are read).
+  int2* ring2 = reinterpret_cast<int2*>(a.ring);
+  uint32_t at = 0;  // the line's slot of the step at hand
+  auto take = [&](int2 (&in)[W], int2 (&acc)[W]) {
+#pragma unroll
+    for (uint32_t k = 0; k < W; ++k) {
+      in[k] = make_int2(0, 0);
+      if (rd[k]) in[k] = __ldcg(ring2 + (slot * a.n_pad + i[k]));
     }
-    uint32_t sp = __ballot_sync(kFull, hit);
-    while (sp) {
-      const int src = __ffs(sp) - 1;
-      sp &= sp - 1;
-      const uint4 h = s_sh[wib * 32u + src];
-      walked += push_any<BF16>(a, s_rows, make_uint2(h.y, h.z), ix.slot, prev);
+#pragma unroll
+    for (uint32_t k = 0; k < W; ++k) {
+      acc[k] = in[k];
+      if (heavy && rd[k]) {
+        int2* p = s_line + at * n_cell + cell[k];
+        const int2 l = *p;
+        if (l.x | l.y) *p = make_int2(0, 0);
+        acc[k] = make_int2(in[k].x + l.x, in[k].y + l.y);
+      }
     }
+  };
+  auto clear_in = [&](uint32_t from, const int2 (&in)[W]) {
+#pragma unroll
+    for (uint32_t k = 0; k < W; ++k)
+      if (in[k].x | in[k].y) __stcg(ring2 + (from * a.n_pad + i[k]), make_int2(0, 0));
+  };
+  auto next_step = [&]() {
+    at = at + 1u == n_line ? 0u : at + 1u;
+    slot = slot + 1u == a.ring_slots ? 0u : slot + 1u;
   };
   if (TL == 0) {
-    // Step t: update (ring slot t), spikes of t, their pushes and the shards
-    // of step t - 1's spikes; one grid barrier.
+    // Step t: update (slot t), spikes of t, their pushes; one grid barrier.
     for (uint32_t s = 0; s < n_steps; ++s) {
-      ix.t = t0 + s;
-      ix.rel = s;
-      const uint32_t par = s & 1u;
-      clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
-      // Shards of the previous step's spikes (none at a launch's first step:
-      // each launch pushes its last step's shards itself, after the loop).
-      const bool sh_ck = s > 0 && threadIdx.x < n_sh;
-      const uint32_t sh_w =
-          sh_ck ? __ldcg(hist_base(a, ix.hrow) + a.n_words + (s_sh[threadIdx.x].x >> 5)) : 0u;
-      off = nit = 0;
-      if (has) {
-        const bool fired = lif ? cell_fire(a, segs[seg], i, 0u, valid, st, 0u, ix) : next_in;
-        publish(fired, ix, s, par);
+      clear_summary(s + 1u, blockIdx.x * n_thr + threadIdx.x, gridDim.x * n_thr);
+      if (wib < nwk) {
+        uint32_t fired = next_in;
+        int2 in[W], acc[W];
+        take(in, acc);
+        clear_in(slot, in);
+#pragma unroll
+        for (uint32_t k = 0; k < W; ++k)
+          if (lif[k] && lif_step(lif_k(segs[seg[k]]), a.substeps, st[k], acc[k]) && valid[k]) fired |= 1u << k;
+        publish(fired, s, slot);
       }
-      const uint32_t sh_from = shard_items(sh_ck, sh_w, par);
-      deliver(par, ix.slot, ix.slot == 0u ? a.ring_slots - 1u : ix.slot - 1u, sh_from);
+      deliver(s & 1u, slot, n_wrp);
       grid_arrive(a, target);
-      if (stim && s + 1 < n_steps)
-        next_in = input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), ix.t + 1);
-      if (!grid_wait(a, target, s_poller)) {
+      if (stim && s + 1 < n_steps) next_in = s == 0u ? next1 : draw(t0 + s + 1ull);
+      if (wib == aide) {
+        if (heavy) board(s, at);
+        if (shared_on) sources(t0 + s + 2ull);
+      }
+      next_step();
+      if (!grid_wait(a, target, last * 32u) || !s_board_ok) {
         aborted = true;
         break;
       }
-      ix_advance(a, ix);
     }
-    // The shards of the last step's spikes (ix has advanced past that step).
-    if (!aborted && n_sh && n_steps) last_shards();
-  } else if (TL == 1) {
-    // Late-push timeline (one substep per step).  A cell's spike of step t + 1
+  } else {
+    // Late-push timelines (one substep per step).  A cell's spike of step t + 1
     // is decided by its potential after the update of step t (the spike test
     // reads the potential before the step's integration), so step t updates
     // with ring slot t and publishes the spikes of t + 1, whose pushes target
-    // slots t + 2 and later.  Those pushes are first read after the barrier of
-    // step t + 1, so a block arrives at step t's barrier as soon as its cells
-    // are updated, and only then makes the step's writes -- the clears of the
-    // slot it consumed, the history words, counts and pushes of the new
-    // spikes, the shards of step t - 1's spikes (delays >= 3) -- while the
-    // other blocks arrive: the next arrival's release carries them.
-    //   Slot t + 1 is complete at step t + 1's start: own pushes into it come
-    // from steps <= t - 1, shards from steps <= t - 1 as well (a shard reads
-    // the spike of step T in the history row written in step T - 1 and pushes
-    // in step T + 1).  A clear made after step t's arrival is ordered before
-    // the pushes of step t + 2 and later only; with max_delay + 3 ring slots
-    // no push of step t + 1 targets slot t again.  A prologue publishes and
-    // pushes the spikes of the launch's first step; the last step publishes
-    // nothing, so a launch ends in the same state as with the other timelines.
-    //   A warp 31 without a word of its own arrives and polls while the other
-    // 31 warps make the step's writes (they meet on block barrier 1), so the
-    // arrival's release stalls no warp with work; otherwise thread 0 arrives
-    // and the block's poller polls after the writes.
-    int2* ring2 = reinterpret_cast<int2*>(a.ring);
-    const bool rd = has && lif && valid;
-    const bool sync_idle = 31u * gridDim.x + blockIdx.x >= a.n_upd_words;  // block-uniform
-    const uint32_t nw = sync_idle ? kPersistBlock / 32 - 1u : kPersistBlock / 32;
-    __shared__ int s_ok1[2];
-    bool in_next = false;  // input spike of step t + 1, drawn a step ahead
-    if (n_steps) {
-      if (stim && n_steps > 1)
-        in_next = input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), t0 + 1);
-      ix.rel = 0;
-      clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
-      off = nit = 0;
-      if (has) publish(valid && (lif ? st.x > segs[seg].Vth : next_in), ix, 0u, 0u);
-      deliver(0u, ix.slot, ix.slot, kNoRow);
-      grid_arrive(a, target);
-      aborted = !grid_wait(a, target, s_poller);
-    }
-    for (uint32_t s = 0; s < n_steps && !aborted; ++s) {
-      const bool more = s + 1u < n_steps;
-      int2 acc = make_int2(0, 0);
-      if (rd) acc = __ldcg(ring2 + (ix.roff + i));
-      const uint32_t consumed = ix.roff;
-      // Shards of step t - 1's spikes (none at a launch's first step: the
-      // previous launch pushed them after its loop).
-      const bool sh_ck = s > 0 && threadIdx.x < n_sh;
-      const uint32_t sh_w =
-          sh_ck ? __ldcg(hist_base(a, ix.hrow) + a.n_words + (s_sh[threadIdx.x].x >> 5)) : 0u;
-      const uint32_t shard_slot = ix.slot == 0u ? a.ring_slots - 1u : ix.slot - 1u;
-      // From here on ix is step t + 1, whose spikes this step publishes.
-      ix.t += 1ull;
-      ix.rel = s + 1u;
-      ix_advance(a, ix);
-      clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x,
-                         gridDim.x * kPersistBlock);  // the row of step t + 2
-      bool fired = false;
-      if (has) {
-        if (lif) {
-          const LifK k = lif_k(segs[seg]);
-          if (rd) lif_update<1>(k, 1, st, acc);
-          fired = valid && st.x > k.Vth;
-        } else {
-          fired = in_next;
+    // slots t + 2 and later: they are first read after the barrier of step
+    // t + 1.
+    //   TL 1: a block arrives at step t's barrier as soon as its cells are
+    // updated, and only then makes the step's writes -- the clears of the slot
+    // it consumed, the history words, counts and pushes of the new spikes --
+    // while the other blocks arrive: the next arrival's release carries them.
+    // A clear made after step t's arrival is ordered before the pushes of step
+    // t + 2 and later only; with max_delay + 3 ring slots no push of step t + 1
+    // targets slot t again.
+    //   TL 2: every write of step t is first read in step t + 2, so the barrier
+    // is split: at the top of step t + 1, after the block barrier that ends
+    // step t, the last warp fences the block's writes of step t and arrives;
+    // the block waits for the other blocks' arrivals only at the end of step
+    // t + 1, before step t + 2 reads slot t + 2.  Arrival, fence and barrier
+    // latency overlap a step's work, and blocks run at most one step apart:
+    // the last warp clears the summary row of step t + 2 at the top of step t,
+    // before its fence (its bits are set in step t + 1), and the raster
+    // records of neighbouring steps may interleave (each record carries its
+    // step mod 4).
+    //   The last warp arrives and polls while the others work (they meet on block
+    // barrier 1), so the arrival's release stalls no warp with work.
+    // The prologue is the loop's round s = -1: it only publishes and pushes.
+    uint32_t in_next = next_in;  // input spikes of step t + 1, drawn a step ahead
+    if (TL == 2) clear_summary(1u, blockIdx.x * n_thr + threadIdx.x, gridDim.x * n_thr);
+#pragma unroll 1
+    for (int s = -1; s < (int)n_steps; ++s) {
+      const uint32_t rel = (uint32_t)(s + 1);  // the chunk step whose spikes this round publishes
+      const bool more = rel < n_steps;
+      if (s < 0 && !more) break;
+      int2 in[W];
+      const uint32_t consumed = slot;
+      uint32_t fired = in_next;
+      if (s >= 0) {
+        target += gridDim.x;
+        if (TL == 2 && wib == last) {
+          clear_summary(rel + 1u, blockIdx.x * 32u + lane, gridDim.x * 32u);
+          __syncwarp();
+          if (lane == 0) grid_arrive_fenced(a);
+          __syncwarp();
         }
       }
-      __syncthreads();  // the block's updates (and the previous step's writes) are done
-      target += gridDim.x;
-      if (sync_idle && wib == 31u) {
-        if (lane == 0) {
-          asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(a.bar) : "memory");
-          s_ok1[s & 1u] = poll_arrivals(a, target);
+      if (wib < nwk) {
+        int2 acc[W];
+        if (s >= 0) take(in, acc);
+        LifK c = lif_k(segs[seg[0]]);
+#pragma unroll
+        for (uint32_t k = 0; k < W; ++k) {
+          if (k && seg[k] != seg[0]) c = lif_k(segs[seg[k]]);
+          if (s >= 0 && rd[k]) lif_update<1>(c, 1, st[k], acc[k]);
+          if (rd[k] && st[k].x > c.Vth) fired |= 1u << k;
         }
-        __syncwarp();
-      } else {
-        if (!sync_idle && threadIdx.x == 0)
-          asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(a.bar) : "memory");
-        if (rd && (acc.x | acc.y)) __stcg(ring2 + (consumed + i), make_int2(0, 0));
-        const uint32_t par = (s + 1u) & 1u;
-        off = nit = 0;
-        if (has && more) publish(fired, ix, s + 1u, par);
-        const uint32_t sh_from = shard_items(sh_ck, sh_w, par);
-        deliver(par, ix.slot, shard_slot, sh_from, nw);
-        if (stim && s + 2u < n_steps)
-          in_next = input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), ix.t + 1ull);
-        if (!sync_idle && threadIdx.x == s_poller) s_ok1[s & 1u] = poll_arrivals(a, target);
       }
-      __syncthreads();
-      if (!s_ok1[s & 1u]) {
+      const uint32_t line_at = at;
+      if (s >= 0) next_step();  // from here on slot and at are those of step `rel`
+      if (TL == 1) {
+        clear_summary(rel + 1u, blockIdx.x * n_thr + threadIdx.x, gridDim.x * n_thr);
+        __syncthreads();  // the block's updates (and the previous step's writes) are done
+        if (s >= 0 && threadIdx.x == last * 32u)
+          asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(a.bar) : "memory");
+      }
+      if (wib < nw) {
+        if (wib < nwk) {
+          if (s >= 0) clear_in(consumed, in);
+          if (more) publish(fired, rel, slot);
+        }
+        deliver(rel & 1u, slot, nw);
+        if (stim && rel + 1u < n_steps) in_next = s < 0 ? next1 : draw(t0 + rel + 1ull);
+      }
+      if (wib == aide) {
+        if (heavy && s >= 0) board((uint32_t)s, line_at);
+        if (shared_on) sources(t0 + rel + 2ull);
+      }
+      if (s < 0) {
+        if (TL == 1) {
+          grid_arrive(a, target);  // with the prologue's writes, before the first update's
+          if (threadIdx.x == last * 32u) s_ok[rel & 1u] = poll_arrivals(a, target);
+        } else if (threadIdx.x == 0) {
+          s_ok[rel & 1u] = 1;
+        }
+      } else if (threadIdx.x == last * 32u) {
+        // A board that ran out of time ends the launch here or a round later.
+        s_ok[rel & 1u] = poll_arrivals(a, target) && *(volatile int*)&s_board_ok;
+      }
+      __syncthreads();  // ends the step: the next arrival's release carries its writes
+      if (!s_ok[rel & 1u]) {
         aborted = true;
         break;
       }
     }
-    // The shards of the last step's spikes (ix has advanced past that step).
-    if (!aborted && n_sh && n_steps) last_shards();
-  } else {
-    // Late-push timeline with a split grid barrier (one substep per step).
-    // The steps' work and data as in the timeline above, but every write of
-    // step t is first read in step t + 2, so the barrier is split: at the top
-    // of step t + 1, after the block barrier that ends step t, warp 31 fences
-    // the block's writes of step t and arrives; the block waits for the other
-    // blocks' arrivals only at the end of step t + 1, before step t + 2 reads
-    // slot t + 2.  Arrival, fence and barrier latency overlap a step's work,
-    // and blocks run at most one step apart, which adds to the timeline above:
-    //   * a history row is rewritten hist_rows steps later: with shards the
-    //     handle keeps at least 4 rows, so that no block rewrites a row before
-    //     a block one step behind has read it for its shards;
-    //   * warp 31 clears the summary row of step t + 2 at the top of step t,
-    //     before its fence; its bits are set in step t + 1;
-    //   * the raster records of neighbouring steps may interleave (each
-    //     record carries its step mod 4).
-    // A warp 31 without a word of its own polls right after arriving while
-    // the other 31 warps work (they meet on block barrier 1); one with a word
-    // works like the others and the block's poller polls at the end.
-    int2* ring2 = reinterpret_cast<int2*>(a.ring);
-    const bool rd = has && lif && valid;
-    const bool sync_idle = 31u * gridDim.x + blockIdx.x >= a.n_upd_words;  // block-uniform
-    const uint32_t nw = sync_idle ? kPersistBlock / 32 - 1u : kPersistBlock / 32;
-    __shared__ int s_ok[2];
-    bool in_next = false;  // input spike of step t + 1, drawn a step ahead
-    if (n_steps) {
-      // Prologue: the spikes of the launch's first step, published and pushed
-      // (fenced with the first arrival, read from step t0 + 1 on).
-      if (stim && n_steps > 1)
-        in_next = input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), t0 + 1);
-      ix.rel = 0;
-      clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
-      off = nit = 0;
-      if (has) publish(valid && (lif ? st.x > segs[seg].Vth : next_in), ix, 0u, 0u);
-      deliver(0u, ix.slot, ix.slot, kNoRow);
-      __syncthreads();
-    }
-    for (uint32_t s = 0; s < n_steps; ++s) {
-      const bool more = s + 1u < n_steps;
-      target += gridDim.x;
-      if (wib == 31u) {
-        const uint32_t row = (ix.srow + 2u) % (a.hist_rows + 1u);  // summary row of step t + 2
-        for (uint32_t j = blockIdx.x * 32u + lane; j < a.n_swords; j += gridDim.x * 32u)
-          __stcg(a.hsum + (size_t)row * a.n_swords + j, 0u);
-        __syncwarp();
-        if (lane == 0) {
-          grid_arrive_fenced(a);
-          if (sync_idle) s_ok[s & 1u] = poll_arrivals(a, target);
-        }
-        __syncwarp();
-      }
-      if (!sync_idle || wib != 31u) {
-        int2 acc = make_int2(0, 0);
-        if (rd) acc = __ldcg(ring2 + (ix.roff + i));
-        const uint32_t consumed = ix.roff;
-        // Shards of step t - 1's spikes (none at a launch's first step: the
-        // previous launch pushed them after its loop).
-        const bool sh_ck = s > 0 && threadIdx.x < n_sh;
-        const uint32_t sh_w =
-            sh_ck ? __ldcg(hist_base(a, ix.hrow) + a.n_words + (s_sh[threadIdx.x].x >> 5)) : 0u;
-        const uint32_t shard_slot = ix.slot == 0u ? a.ring_slots - 1u : ix.slot - 1u;
-        // From here on ix is step t + 1, whose spikes this step publishes.
-        ix.t += 1ull;
-        ix.rel = s + 1u;
-        ix_advance(a, ix);
-        bool fired = false;
-        if (has) {
-          if (lif) {
-            const LifK k = lif_k(segs[seg]);
-            if (rd) lif_update<1>(k, 1, st, acc);
-            fired = valid && st.x > k.Vth;
-          } else {
-            fired = in_next;
-          }
-        }
-        if (rd && (acc.x | acc.y)) __stcg(ring2 + (consumed + i), make_int2(0, 0));
-        const uint32_t par = (s + 1u) & 1u;
-        off = nit = 0;
-        if (has && more) publish(fired, ix, s + 1u, par);
-        const uint32_t sh_from = shard_items(sh_ck, sh_w, par);
-        deliver(par, ix.slot, shard_slot, sh_from, nw);
-        if (stim && s + 2u < n_steps)
-          in_next = input_fire(a, srcs, segs[seg], __float_as_uint(st.y), __float_as_uint(st.x), ix.t + 1ull);
-        if (!sync_idle && threadIdx.x == s_poller) s_ok[s & 1u] = poll_arrivals(a, target);
-      } else {
-        ix.t += 1ull;
-        ix.rel = s + 1u;
-        ix_advance(a, ix);
-      }
-      __syncthreads();  // ends the step: the next arrival fences its writes
-      if (!s_ok[s & 1u]) {
-        aborted = true;
-        break;
-      }
-    }
-    // The shards of the last step's spikes (ix has advanced past that step).
-    if (!aborted && n_sh && n_steps) last_shards();
   }
-  if (valid && lif) state_out(a, i, st);
+  // The line's pending increments (steps t0 + n_steps and later) into the ring.
+  if (heavy && !aborted) {
+#pragma unroll 1
+    for (uint32_t d = 0; d < a.max_delay; ++d) {
+#pragma unroll
+      for (uint32_t k = 0; k < W; ++k) {
+        if (!rd[k]) continue;
+        const int2 l = s_line[at * n_cell + cell[k]];
+        int* p = a.ring + (((size_t)slot * a.n_pad + i[k]) << 1);
+        if (l.x) atomicAdd(p, l.x);
+        if (l.y) atomicAdd(p + 1, l.y);
+      }
+      next_step();
+    }
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < W; ++k)
+    if (rd[k]) state_out(a, i[k], st[k]);
   if (a.raster_cap && blockIdx.x == 0) raster_offsets_from_counts(a, n_steps, s_wsum);
   if (__ldcg(&ctl->error) & kErrBarrierTimeout) return;
   if (lane == 0 && walked) atomicAdd(&ctl->delivered, (unsigned long long)walked);
   if (leader) {
     ctl->step = t0 + n_steps;
-    ctl->ring_slot = ix.slot;
-    ctl->hist_row = ix.hrow;
+    ctl->ring_slot = (ix0.slot + n_steps) % a.ring_slots;
+    ctl->hist_row = (ix0.hrow + n_steps) % n_hist;
     ctl->t_rel = n_steps;
   }
 }
@@ -2678,16 +2797,31 @@ cudaError_t launch_chunk_end(const StepArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// The fused kernel's forms: [BF16][0: spikes in their own step, 64-synapse
-// items; 1, 2: late-push timeline, 3, 4: late push with the split barrier,
-// each with items of 64 and 128 synapses].
-#define SGB_FUSED_FORMS(B)                                                                  \
-  (const void*)k_persistent_fused<B, 0, 6>, (const void*)k_persistent_fused<B, 1, 6>,        \
-      (const void*)k_persistent_fused<B, 1, 7>, (const void*)k_persistent_fused<B, 2, 6>,    \
-      (const void*)k_persistent_fused<B, 2, 7>
-constexpr uint32_t kFusedForms = 5;
+// The fused kernel's forms: [BF16][timeline][words per warp - 1].
+#define SGB_FUSED_FORMS(B)                                                      \
+  (const void*)k_persistent_fused<B, 0, 1>, (const void*)k_persistent_fused<B, 0, 2>,     \
+      (const void*)k_persistent_fused<B, 1, 1>, (const void*)k_persistent_fused<B, 1, 2>, \
+      (const void*)k_persistent_fused<B, 2, 1>, (const void*)k_persistent_fused<B, 2, 2>
+constexpr uint32_t kFusedForms = 6;
 static const void* const kFusedKernels[] = {SGB_FUSED_FORMS(false), SGB_FUSED_FORMS(true)};
 #undef SGB_FUSED_FORMS
+
+// Words per block, at most, and per warp: a warp without a word still runs a
+// step's bookkeeping, and in steps bound by latency those instructions delay
+// the warps with work, so blocks are no larger than needed (9,256 cells, two
+// words a block: 1.73 us per step with 32 warps, 1.58 with 8).
+static uint32_t fused_words(const StepArgs& a, int blocks) {
+  return (a.n_upd_words + (uint32_t)blocks - 1u) / (uint32_t)blocks;
+}
+static uint32_t fused_per_warp(const StepArgs& a, int blocks) {
+  return fused_words(a, blocks) <= kFusedSingle ? 1u : 2u;
+}
+constexpr uint32_t kFusedWarps = 8;  // at least
+static uint32_t fused_threads(const StepArgs& a, int blocks) {
+  const uint32_t w = fused_per_warp(a, blocks);
+  return 32u * std::max((fused_words(a, blocks) + w - 1u) / w + 2u, kFusedWarps);
+}
+size_t fused_heavy_bytes(const StepArgs& a, int blocks) { return hv_bytes(a, (uint32_t)blocks); }
 
 // The timeline and item width the fused kernel runs with for these arguments.
 uint32_t fused_timeline(const StepArgs& a) { return a.substeps == 1 ? std::min(a.ahead, 2u) : 0u; }
@@ -2695,17 +2829,15 @@ uint32_t fused_item_log2(const StepArgs& a) {
   return fused_timeline(a) ? (a.item_log2 >= 7 ? 7u : 6u) : 6u;
 }
 
-static const void* fused_kernel(const StepArgs& a) {
-  const uint32_t tl = fused_timeline(a);
-  const uint32_t form = tl ? 2u * tl - 1u + (fused_item_log2(a) - 6u) : 0u;
-  return kFusedKernels[(a.bf16 ? kFusedForms : 0u) + form];
+static const void* fused_kernel(const StepArgs& a, int blocks) {
+  return kFusedKernels[(a.bf16 ? kFusedForms : 0u) + 2u * fused_timeline(a) + fused_per_warp(a, blocks) - 1u];
 }
 
 static int fused_blocks_per_sm() {
   int n = 1 << 20;
-  for (const void* fn : kFusedKernels) {
+  for (uint32_t k = 0; k < 2u * kFusedForms; ++k) {
     int f = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, fn, kPersistBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, kFusedKernels[k], (int)fused_max_threads(k % 2u + 1u), 0);
     n = f < n ? f : n;
   }
   return n;
@@ -2783,7 +2915,7 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
                                        dim3(pull_threads(a, blocks)), params, a.pull_smem, s);
   const bool resident = kind != SGB_KERNEL_GENERAL;
   const bool fused = kind == SGB_KERNEL_FUSED;
-  const void* fn = fused      ? fused_kernel(a)
+  const void* fn = fused      ? fused_kernel(a, blocks)
                    : resident ? (a.bf16 ? (const void*)k_persistent_resident<true>
                                         : (const void*)k_persistent_resident<false>)
                    : general_one_barrier(a)
@@ -2797,7 +2929,8 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
   const size_t smem = fused ? a.row_smem
                      : (a.seg_smem ? seg_smem_bytes(a) : 0) +
                            ((a.n_pull_units && a.pull_sum) ? pull_sum_bytes(a) : 0);
-  return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kPersistBlock), params, smem, s);
+  const uint32_t threads = fused ? fused_threads(a, blocks) : kPersistBlock;
+  return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), params, smem, s);
 }
 
 uint32_t fused_row_smem_max() {
