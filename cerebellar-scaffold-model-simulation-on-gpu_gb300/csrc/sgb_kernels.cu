@@ -57,6 +57,7 @@ struct StepIdx {
   uint32_t roff;   // ring slot: slot * n_pad (int2 elements)
   uint32_t hoff;   // history row of step t: (hist_rows - 1 - hrow) * n_words
   uint32_t hoff2;  // its second copy, hist_rows rows further
+  bool keep;       // general kernel, two cells per lane: write the history row
 };
 
 template <bool BF16>
@@ -451,29 +452,33 @@ __device__ __forceinline__ void put_hist2(const StepArgs& a, const StepIdx& ix, 
   if (sbits) atomicOr(a.hsum + (size_t)ix.srow * a.n_swords + (w >> 5), sbits);
 }
 
-// Spike bookkeeping of a pair: bitmap words, per-segment counts (one per
-// word), events, raster entries, and the spiking cells' push rows cut into
-// kPushChunk items in the block's list (items past its capacity are pushed
-// here).  Returns the synapses pushed here.
+// Spike bookkeeping of a pair: per-segment counts (one per word), events,
+// raster entries, and the spiking cells' push rows cut into kPushChunk items
+// in the block's list (items past its capacity are pushed here); with ix.keep
+// also the bitmap words.  Returns the synapses pushed here.  Without the
+// history of every step and the scans over the warp (a lane reserves its own
+// items): 925,500 cells 8.2 -> 7.6 us per step, 32 instances with 3.3M cells
+// 18.9 -> 17.3 us.
 template <bool BF16>
 __device__ __forceinline__ uint32_t publish_pair(const StepArgs& a, uint32_t p, uint32_t c,
                                                  uint32_t seg, bool f0, bool f1, const StepIdx& ix,
                                                  BlockItems bi) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t packed = (f0 ? 1u : 0u) | (f1 ? 2u : 0u);
-  // Cell j of word 2p is lane j >> 1's cell j & 1; of word 2p + 1, lane 16 + (j >> 1)'s.
-  const uint32_t x0 = __shfl_sync(kFull, packed, lane >> 1);
-  const uint32_t x1 = __shfl_sync(kFull, packed, 16u + (lane >> 1));
-  const uint32_t W0 = __ballot_sync(kFull, (x0 >> (lane & 1u)) & 1u);
-  const uint32_t W1 = __ballot_sync(kFull, (x1 >> (lane & 1u)) & 1u);
-  if (lane == 0) put_hist2(a, ix, 2u * p, W0, W1);
-  if ((W0 | W1) == 0u) return 0;
+  const uint32_t b0 = __ballot_sync(kFull, f0), b1 = __ballot_sync(kFull, f1);
+  if (ix.keep) {
+    // Cell j of word 2p is lane j >> 1's cell j & 1; of word 2p + 1, lane 16 + (j >> 1)'s.
+    const uint32_t from = (lane & 1u) ? b1 : b0;
+    const uint32_t W0 = __ballot_sync(kFull, (from >> (lane >> 1)) & 1u);
+    const uint32_t W1 = __ballot_sync(kFull, (from >> (16u + (lane >> 1))) & 1u);
+    if (lane == 0) put_hist2(a, ix, 2u * p, W0, W1);
+  }
+  if ((b0 | b1) == 0u) return 0;
   Ctl* ctl = a.ctl;
-  const uint32_t mine = lane < 16u ? W0 : W1;
-  if ((lane & 15u) == 0u && mine)
-    atomicAdd(&a.counts[(size_t)ix.rel * a.n_segs + seg], (uint32_t)__popc(mine));
+  const uint32_t half = lane < 16u ? 0xFFFFu : 0xFFFF0000u;  // the lanes of this lane's word
+  const uint32_t mine = __popc(b0 & half) + __popc(b1 & half);
+  if ((lane & 15u) == 0u && mine) atomicAdd(&a.counts[(size_t)ix.rel * a.n_segs + seg], mine);
   uint32_t ev = 0, ra = 0, rb = 0, rc = 0;
-  if (packed) {
+  if (f0 || f1) {
     if (f0) ev += __ldg(a.outdeg + c);
     if (f1) ev += __ldg(a.outdeg + c + 1u);
     if (a.any_push) {
@@ -482,34 +487,17 @@ __device__ __forceinline__ uint32_t publish_pair(const StepArgs& a, uint32_t p, 
       rc = __ldg(a.push_row + c + 2u);
     }
   }
-  ev = __reduce_add_sync(kFull, ev);
   const uint32_t na = f0 ? (rb - ra + kPushChunk - 1) / kPushChunk : 0u;
   const uint32_t nb = f1 ? (rc - rb + kPushChunk - 1) / kPushChunk : 0u;
   const uint32_t nit = na + nb;
-  uint32_t incl = nit;
-  uint32_t rk = (f0 ? 1u : 0u) + (f1 ? 1u : 0u), rincl = rk;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(kFull, incl, o);
-    const uint32_t r = __shfl_up_sync(kFull, rincl, o);
-    if (lane >= (uint32_t)o) {
-      incl += v;
-      rincl += r;
-    }
-  }
-  const uint32_t tot_items = __shfl_sync(kFull, incl, 31);
-  uint32_t off = 0, roff = 0;
-  if (lane == 0) {
-    if (tot_items) off = atomicAdd(bi.count, tot_items);
-    if (ev) atomicAdd(&ctl->events, (unsigned long long)ev);
-    if (a.raster_cap) roff = atomicAdd(&ctl->raster_count, (uint32_t)(__popc(W0) + __popc(W1)));
-  }
-  off = __shfl_sync(kFull, off, 0) + incl - nit;
+  uint32_t off = 0;
+  if (nit) off = atomicAdd(bi.count, nit);
   for (uint32_t k = 0; k < nit && off + k < kGenItems; ++k) {
     const uint32_t q0 = k < na ? ra + k * kPushChunk : rb + (k - na) * kPushChunk;
     const uint32_t q1 = k < na ? rb : rc;
     bi.items[off + k] = make_uint2(q0, min(kPushChunk, q1 - q0) << 23);
   }
+  if (ev) atomicAdd(&ctl->events, (unsigned long long)ev);
   uint32_t walked = 0;
   uint32_t spill = __ballot_sync(kFull, off + nit > kGenItems);
   while (spill) {
@@ -526,8 +514,10 @@ __device__ __forceinline__ uint32_t publish_pair(const StepArgs& a, uint32_t p, 
     }
   }
   if (a.raster_cap) {
-    roff = __shfl_sync(kFull, roff, 0) + rincl - rk;
-    uint32_t q = roff;
+    uint32_t roff = 0;
+    if (lane == 0) roff = atomicAdd(&ctl->raster_count, (uint32_t)(__popc(b0) + __popc(b1)));
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t q = __shfl_sync(kFull, roff, 0) + __popc(b0 & below) + __popc(b1 & below);
     if (f0) {
       if (q < a.raster_cap) a.raster[q] = c; else atomicOr(&ctl->error, kErrRasterOverflow);
       ++q;
@@ -1369,7 +1359,13 @@ __global__ void __launch_bounds__(kPersistBlock, 1) k_persistent(StepArgs a, uin
     // Item counter of step t + 1: its last user was the update of step t - 1
     // (kept zero in ONE launches too, for launches of the other form).
     if (leader) __stcg(&ctl->active_count[(ix.t + 1) & 1], 0u);
-    clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
+    // Without dense pulls and plasticity no one reads the history during the
+    // launch: it writes the rows of its last hist_rows steps, for the other
+    // kernels and the host, and clears their summary rows and the next one's.
+    const bool all_rows = LANE != 2;
+    ix.keep = all_rows || s + a.hist_rows >= n_steps;
+    if (all_rows || s + 1u + a.hist_rows >= n_steps)
+      clear_next_summary(a, ix, blockIdx.x * kPersistBlock + threadIdx.x, gridDim.x * kPersistBlock);
     const BlockItems bi{s_items, &s_icnt[s & 1u]};
     if (a.n_plast)
       walked += a.seg_smem ? update_words<true, true, BF16, ONE>(a, uw, nw, ix, bi)
