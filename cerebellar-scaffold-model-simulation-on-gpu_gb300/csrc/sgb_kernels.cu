@@ -769,6 +769,18 @@ __device__ __forceinline__ void ix_advance(const StepArgs& a, StepIdx& ix) {
 }
 
 // ---- per-step kernels (CUDA-graph driver) ----------------------------------
+// A step's kernels depend on one another, but their launches need not: each is
+// launched as a programmatic dependent of the one before (step_launch), so its
+// blocks are scheduled while that one still runs, and waits here before its
+// first access for that kernel to end and its writes to be visible.  Every
+// block passes this point, so a kernel's end implies the end of all before it.
+// In a graph: 92,550 cells event-driven 6.85 -> 6.5 us per step, every
+// projection dense 13.3 -> 12.2, 9,255 cells 5.8 -> 5.4.
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __global__ void k_chunk_begin(StepArgs a) {
   a.ctl->t_rel = 0;
   a.ctl->raster_count = 0;
@@ -776,6 +788,7 @@ __global__ void k_chunk_begin(StepArgs a) {
 }
 
 __global__ void __launch_bounds__(kBlock) k_update(StepArgs a) {
+  step_begin();
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t w = gtid >> 5;
   const StepIdx ix = step_of(a);
@@ -788,6 +801,7 @@ __global__ void __launch_bounds__(kBlock) k_update(StepArgs a) {
 // (ring slot, history row, buffer parity, raster offsets).
 template <bool BF16>
 __global__ void __launch_bounds__(kBlock) k_deliver(StepArgs a) {
+  step_begin();
   Ctl* ctl = a.ctl;
   const StepIdx ix = step_of(a);
   const uint32_t lane = threadIdx.x & 31u;
@@ -834,6 +848,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) k_pull(StepArgs a) {
   const uint32_t gw = (blockIdx.x * kPullBlock + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * kPullBlock) >> 5;
   const uint32_t n = a.n_pull_units;
+  step_begin();
   const StepIdx ix = step_of(a);
   const uint32_t slot1 = ix.slot + 1u == a.ring_slots ? 0u : ix.slot + 1u;
   uint32_t e[E];
@@ -908,6 +923,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) k_pull_vec(StepArgs a) {
   const uint32_t gw = (blockIdx.x * kPullBlock + threadIdx.x) >> 5;
   const uint32_t nw = (gridDim.x * kPullBlock) >> 5;
   const uint32_t n = a.n_pull_units;
+  step_begin();
   const StepIdx ix = step_of(a);
   const uint32_t slot1 = ix.slot + 1u == a.ring_slots ? 0u : ix.slot + 1u;
   uint4 q[V];
@@ -2670,18 +2686,31 @@ cudaError_t launch_chunk_begin(const StepArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Launches a kernel of a step behind the previous one; without plastic
+// projections (whose plasticity runs on a forked stream) as its programmatic
+// dependent.
+static cudaError_t step_launch(void (*fn)(StepArgs), const StepArgs& a, int blocks, int threads, size_t smem,
+                               cudaStream_t s) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = a.n_plast ? 0 : 1;
+  return cudaLaunchKernelEx(&cfg, fn, a);
+}
+
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s) {
   if (!a.n_upd_words) return cudaSuccess;
-  k_update<<<(a.n_words + kBlock / 32 - 1) / (kBlock / 32), kBlock, 0, s>>>(a);
-  return cudaGetLastError();
+  return step_launch(k_update, a, (a.n_words + kBlock / 32 - 1) / (kBlock / 32), kBlock, 0, s);
 }
 
 cudaError_t launch_deliver(const StepArgs& a, int blocks, cudaStream_t s) {
-  if (a.bf16)
-    k_deliver<true><<<blocks, kBlock, 0, s>>>(a);
-  else
-    k_deliver<false><<<blocks, kBlock, 0, s>>>(a);
-  return cudaGetLastError();
+  return step_launch(a.bf16 ? k_deliver<true> : k_deliver<false>, a, blocks, kBlock, 0, s);
 }
 
 size_t pull_sum_bytes(const StepArgs& a) { return ((size_t)a.hist_rows * a.n_swords + 1) * 4; }
@@ -2691,21 +2720,11 @@ static size_t pull_smem_bytes(const StepArgs& a) { return a.pull_sum ? pull_sum_
 
 cudaError_t launch_pull(const StepArgs& a, int blocks, cudaStream_t s) {
   if (!a.n_pull_units) return cudaSuccess;
-  if (a.pull_sum == 2u) {
-    const size_t smem = pull_sum_bytes(a);
-    if (a.bf16) k_pull_vec<true><<<blocks, kPullBlock, smem, s>>>(a);
-    else k_pull_vec<false><<<blocks, kPullBlock, smem, s>>>(a);
-    return cudaGetLastError();
-  }
-  const size_t smem = pull_smem_bytes(a);
-  if (a.bf16) {
-    if (a.pull_sum) k_pull<true, true><<<blocks, kPullBlock, smem, s>>>(a);
-    else k_pull<true, false><<<blocks, kPullBlock, smem, s>>>(a);
-  } else {
-    if (a.pull_sum) k_pull<false, true><<<blocks, kPullBlock, smem, s>>>(a);
-    else k_pull<false, false><<<blocks, kPullBlock, smem, s>>>(a);
-  }
-  return cudaGetLastError();
+  if (a.pull_sum == 2u)
+    return step_launch(a.bf16 ? k_pull_vec<true> : k_pull_vec<false>, a, blocks, kPullBlock, pull_sum_bytes(a), s);
+  void (*fn)(StepArgs) = a.bf16 ? (a.pull_sum ? k_pull<true, true> : k_pull<true, false>)
+                                : (a.pull_sum ? k_pull<false, true> : k_pull<false, false>);
+  return step_launch(fn, a, blocks, kPullBlock, pull_smem_bytes(a), s);
 }
 
 cudaError_t launch_stdp(const StepArgs& a, int blocks, cudaStream_t s, bool early) {
