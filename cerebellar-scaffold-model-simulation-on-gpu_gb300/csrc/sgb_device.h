@@ -229,11 +229,15 @@ struct StepArgs {
 };
 
 // Launch wrappers (sgb_kernels.cu).  All return the launch status.
-cudaError_t launch_chunk_begin(const StepArgs& a, cudaStream_t s);
+// Chunk of `steps` steps: clears its counts and n_bar words from a.bar, and loads
+// the stimulus sources from `srcs` (pinned host memory; NULL: unchanged).
+cudaError_t launch_chunk_begin(const StepArgs& a, uint32_t steps, uint32_t n_bar, const SrcDev* srcs,
+                               cudaStream_t s);
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s);
 // Delivery of the current step; also advances the step counter.
 cudaError_t launch_deliver(const StepArgs& a, int blocks, cudaStream_t s);
-cudaError_t launch_chunk_end(const StepArgs& a, cudaStream_t s);
+// host_err, host_counts: pinned host memory (counts NULL: not wanted).
+cudaError_t launch_chunk_end(const StepArgs& a, uint32_t* host_err, uint32_t* host_counts, cudaStream_t s);
 // One cooperative launch advancing n_steps; grid = blocks (all co-resident).
 cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, cudaStream_t s);
 // Largest dynamic shared memory the fused persistent kernel can take for push

@@ -71,6 +71,7 @@ Sim::~Sim() {
   if (h_raster) cudaFreeHost(h_raster);
   if (h_raster_off) cudaFreeHost(h_raster_off);
   if (h_srcs) cudaFreeHost(h_srcs);
+  if (h_err) cudaFreeHost(h_err);
   if (own_stream) cudaStreamDestroy(own_stream);
 }
 
@@ -832,6 +833,8 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   s.persistent_blocks = std::max(1, bpsm) * s.sm_count;
 
   SGB_CUDA(cudaMemcpy((void*)a.segs, s.segs.data(), nseg * sizeof(SegDev), cudaMemcpyHostToDevice));
+  SGB_CUDA(cudaMallocHost(&s.h_err, sizeof(uint32_t)));
+  *s.h_err = 0;
   SGB_CUDA(cudaMallocHost(&s.h_srcs, std::max<size_t>(s.srcs.size(), 1) * sizeof(SrcDev)));
   if (!s.srcs.empty()) {
     memcpy(s.h_srcs, s.srcs.data(), s.srcs.size() * sizeof(SrcDev));
@@ -884,21 +887,36 @@ int sim_reset(Sim& s, const uint64_t* seeds) {
   SGB_CUDA(cudaMemsetAsync(a.items, 0, (size_t)2 * a.item_cap * sizeof(uint2), s.stream));
   SGB_CUDA(cudaMemsetAsync(a.totals, 0, s.segs.size() * sizeof(double), s.stream));
   SGB_CUDA(cudaStreamSynchronize(s.stream));
+  s.busy = false;
+  *s.h_err = 0;
+  return SGB_OK;
+}
+
+// Changed stimulus sources onto the device, for the launches that do not take
+// them along themselves.
+static int upload_sources(Sim& s) {
+  if (!s.srcs_dirty) return SGB_OK;
+  SGB_CUDA(cudaMemcpyAsync((void*)s.args.srcs, s.h_srcs, s.srcs.size() * sizeof(SrcDev),
+                           cudaMemcpyHostToDevice, s.stream));
+  s.srcs_dirty = false;
+  s.busy = true;
   return SGB_OK;
 }
 
 // ---------------------------------------------------------------------------
 // One chunk of c steps issued on `st` (direct launches; also the body that is
 // captured into a graph).  *nlaunch receives the number of kernel launches.
-static cudaError_t issue_chunk(Sim& s, uint32_t c, cudaStream_t st, int64_t* nlaunch) {
+// srcs, host_counts: as launch_chunk_begin / launch_chunk_end take them.
+static cudaError_t issue_chunk(Sim& s, uint32_t c, cudaStream_t st, int64_t* nlaunch, const SrcDev* srcs,
+                               uint32_t* host_counts) {
   const StepArgs& a = s.args;
   cudaError_t e;
   int64_t L = 0;
-  if ((e = cudaMemsetAsync(a.counts, 0, (size_t)c * a.n_segs * 4, st))) return e;
-  if ((e = launch_chunk_begin(a, st))) return e;
+  const bool persistent = s.cfg.exec_mode == SGB_EXEC_PERSISTENT;
+  const uint32_t n_bar = (uint32_t)(kBarBytes + 4 * kHeavyWords * sizeof(unsigned long long)) / 4;
+  if ((e = launch_chunk_begin(a, c, persistent ? n_bar : 0u, srcs, st))) return e;
   L++;
-  if (s.cfg.exec_mode == SGB_EXEC_PERSISTENT) {
-    if ((e = cudaMemsetAsync(a.bar, 0, kBarBytes + 4 * kHeavyWords * sizeof(unsigned long long), st))) return e;
+  if (persistent) {
     if ((e = launch_persistent(a, c, s.persistent_blocks, st))) return e;
     L++;
   } else {
@@ -928,20 +946,22 @@ static cudaError_t issue_chunk(Sim& s, uint32_t c, cudaStream_t st, int64_t* nla
       L += 2;
     }
   }
-  if ((e = launch_chunk_end(a, st))) return e;
+  if ((e = launch_chunk_end(a, s.h_err, host_counts, st))) return e;
   L++;
   if (nlaunch) *nlaunch = L;
   return cudaSuccess;
 }
 
-static int launch_chunk(Sim& s, uint32_t c) {
+static int launch_chunk(Sim& s, uint32_t c, uint32_t* host_counts = nullptr) {
   int64_t L = 0;
+  s.busy = true;
   if (s.cfg.exec_mode == SGB_EXEC_GRAPH) {
+    if (int rc = upload_sources(s)) return rc;
     auto it = s.graphs.find(c);
     if (it == s.graphs.end()) {
       cudaGraph_t g;
       SGB_CUDA(cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t e = issue_chunk(s, c, s.stream, &L);
+      cudaError_t e = issue_chunk(s, c, s.stream, &L, nullptr, nullptr);
       cudaError_t e2 = cudaStreamEndCapture(s.stream, &g);
       if (e != cudaSuccess)
         return set_error(SGB_ERR_CUDA, "capture of a %u-step chunk failed: %s", c, cudaGetErrorString(e));
@@ -955,18 +975,31 @@ static int launch_chunk(Sim& s, uint32_t c) {
     SGB_CUDA(cudaGraphLaunch(it->second, s.stream));
     L = 2 + 2 * (int64_t)c;
   } else {
-    cudaError_t e = issue_chunk(s, c, s.stream, &L);
+    cudaError_t e = issue_chunk(s, c, s.stream, &L, s.srcs_dirty ? s.h_srcs : nullptr, host_counts);
     if (e != cudaSuccess) return set_error(SGB_ERR_CUDA, "step launch failed: %s", cudaGetErrorString(e));
+    s.srcs_dirty = false;
   }
   s.launches += L;
   return SGB_OK;
 }
 
-static int check_device_error(Sim& s, uint32_t* bits) {
-  uint32_t err = 0;
-  SGB_CUDA(cudaMemcpyAsync(&err, &s.args.ctl->error, 4, cudaMemcpyDeviceToHost, s.stream));
+// Waits for the stream; afterwards the staging buffers are the host's.
+static int wait_stream(Sim& s) {
   SGB_CUDA(cudaStreamSynchronize(s.stream));
-  if (bits) *bits = err;
+  s.busy = false;
+  return SGB_OK;
+}
+
+// The device's error flags up to the last chunk (after waiting for it); set
+// ones are cleared on the device.
+static int take_device_error(Sim& s, uint32_t* bits) {
+  if (s.busy || s.stream != s.own_stream)
+    if (int rc = wait_stream(s)) return rc;
+  *bits = *(volatile uint32_t*)s.h_err;
+  if (*bits) {
+    *s.h_err = 0;
+    SGB_CUDA(cudaMemsetAsync(&s.args.ctl->error, 0, 4, s.stream));
+  }
   return SGB_OK;
 }
 
@@ -983,9 +1016,9 @@ int sim_enqueue(Sim& s, int64_t n_steps) {
 
 int sim_sync(Sim& s) {
   uint32_t err = 0;
-  int rc = check_device_error(s, &err);
+  SGB_CUDA(cudaStreamSynchronize(s.stream));
+  int rc = take_device_error(s, &err);
   if (rc) return rc;
-  SGB_CUDA(cudaMemsetAsync(&s.args.ctl->error, 0, 4, s.stream));
   if (err & kErrBarrierTimeout)
     return set_error(SGB_ERR_DEVICE, "a device-side grid barrier hit its wait limit; reset the handle");
 
@@ -1006,14 +1039,20 @@ int sim_run(Sim& s, int64_t n_steps, uint32_t* counts, uint32_t* raster_ids, int
   if (raster_offsets) raster_offsets[0] = 0;
   while (done < n_steps) {
     const uint32_t c = (uint32_t)std::min<int64_t>(s.chunk, n_steps - done);
-    int rc = launch_chunk(s, c);
+    // Few counts (up to 64 KiB) are written to the host by the chunk's last
+    // kernel: 10 steps with 7 populations, rates set and counts read by the
+    // caller, 82 us per call with copies for sources, counts and flags and
+    // memsets before each launch, 61 us without.
+    const bool direct = counts && s.cfg.exec_mode != SGB_EXEC_GRAPH && (size_t)c * nseg * 4 <= 65536;
+    int rc = launch_chunk(s, c, direct ? s.h_counts : nullptr);
     if (rc) return rc;
     if (counts || want_raster) {
       const StepArgs& a = s.args;
-      SGB_CUDA(cudaMemcpyAsync(s.h_counts, a.counts, (size_t)c * nseg * 4, cudaMemcpyDeviceToHost, s.stream));
+      if (counts && !direct)
+        SGB_CUDA(cudaMemcpyAsync(s.h_counts, a.counts, (size_t)c * nseg * 4, cudaMemcpyDeviceToHost, s.stream));
       if (want_raster)
         SGB_CUDA(cudaMemcpyAsync(s.h_raster_off, a.raster_off, (size_t)(c + 1) * 4, cudaMemcpyDeviceToHost, s.stream));
-      SGB_CUDA(cudaStreamSynchronize(s.stream));
+      if ((rc = wait_stream(s))) return rc;
       if (counts) memcpy(counts + (size_t)done * nseg, s.h_counts, (size_t)c * nseg * 4);
       if (want_raster) {
         const uint32_t nrec = std::min<uint32_t>(s.h_raster_off[c], s.raster_cap);
@@ -1058,9 +1097,8 @@ int sim_run(Sim& s, int64_t n_steps, uint32_t* counts, uint32_t* raster_ids, int
     done += c;
   }
   uint32_t err = 0;
-  int rc = check_device_error(s, &err);
+  int rc = take_device_error(s, &err);
   if (rc) return rc;
-  SGB_CUDA(cudaMemsetAsync(&s.args.ctl->error, 0, 4, s.stream));
   if (err & kErrBarrierTimeout)
     return set_error(SGB_ERR_DEVICE, "a device-side grid barrier hit its wait limit; reset the handle");
 
@@ -1082,11 +1120,15 @@ int sim_set_rates(Sim& s, int32_t net, int32_t n, const float* rates) {
     fill_source(s.srcs[k], p, s.cfg.dt_ms);
   }
   if (!s.srcs.empty()) {
-    // The pinned staging copy is reused only after the previous upload ended.
-    SGB_CUDA(cudaStreamSynchronize(s.stream));
+    // The pinned staging copy is reused only after the chunks that may read it.
+    const bool shared = s.stream != s.own_stream;
+    if (s.busy || shared)
+      if (int rc = wait_stream(s)) return rc;
     memcpy(s.h_srcs, s.srcs.data(), s.srcs.size() * sizeof(SrcDev));
-    SGB_CUDA(cudaMemcpyAsync((void*)s.args.srcs, s.h_srcs, s.srcs.size() * sizeof(SrcDev),
-                             cudaMemcpyHostToDevice, s.stream));
+    s.srcs_dirty = true;
+    // The caller's stream may be capturing the steps, or replaying captured
+    // ones, which must find the new sources in place.
+    if (shared) return upload_sources(s);
   }
   return SGB_OK;
 }
@@ -1235,7 +1277,8 @@ int sim_set_mode(Sim& s, int32_t net, int32_t proj, int32_t mode) {
 }
 
 int sim_set_stream(Sim& s, cudaStream_t st) {
-  SGB_CUDA(cudaStreamSynchronize(s.stream));
+  if (int rc = upload_sources(s)) return rc;
+  if (int rc = wait_stream(s)) return rc;
   cudaStream_t next = st ? st : s.own_stream;
   if (s.l2_window && next != s.stream) {
     // The state window follows the handle's launches; a caller's stream is
@@ -1535,8 +1578,9 @@ int sim_profile(Sim& s, int32_t n_steps, double* mean_us, double* bytes, int64_t
   int32_t done = 0;
   while (done < n_steps) {
     const uint32_t c = (uint32_t)std::min<int64_t>(s.chunk, n_steps - done);
-    SGB_CUDA(cudaMemsetAsync(a.counts, 0, (size_t)c * a.n_segs * 4, s.stream));
-    SGB_CUDA(launch_chunk_begin(a, s.stream));
+    if (int rc = upload_sources(s)) return rc;
+    s.busy = true;
+    SGB_CUDA(launch_chunk_begin(a, c, 0u, nullptr, s.stream));
     for (uint32_t i = 0; i < c; ++i) {
       SGB_CUDA(cudaMemcpyAsync(&before, a.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s.stream));
       SGB_CUDA(cudaEventRecord(ev[0], s.stream));
@@ -1570,7 +1614,7 @@ int sim_profile(Sim& s, int32_t n_steps, double* mean_us, double* bytes, int64_t
         nl[k]++;
       }
     }
-    SGB_CUDA(launch_chunk_end(a, s.stream));
+    SGB_CUDA(launch_chunk_end(a, s.h_err, nullptr, s.stream));
     s.launches += 2;
     done += (int32_t)c;
   }
@@ -1702,6 +1746,7 @@ int sim_checkpoint(Sim& s, void* buf, int64_t size, bool load) {
     if (nsrc) {
       memcpy(s.srcs.data(), p, nsrc);
       memcpy(s.h_srcs, s.srcs.data(), nsrc);
+      s.srcs_dirty = false;
       SGB_CUDA(cudaMemcpy((void*)s.args.srcs, s.h_srcs, nsrc, cudaMemcpyHostToDevice));
     }
   } else if (nsrc) {

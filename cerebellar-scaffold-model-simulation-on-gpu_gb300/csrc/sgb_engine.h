@@ -84,6 +84,9 @@ struct Sim {
   size_t l2_window = 0, l2_setaside = 0, l2_prev_limit = 0;
   float l2_hit = 0.f;
   SrcDev* h_srcs = nullptr;  // pinned staging of the source table
+  bool srcs_dirty = false;   // h_srcs not yet on the device: the next chunk takes it along
+  bool busy = false;         // work that may read h_srcs has been issued since the last wait
+  uint32_t* h_err = nullptr; // pinned: the device's error flags at the end of the last chunk
 
   // Host staging for outputs.
   uint32_t* h_counts = nullptr;

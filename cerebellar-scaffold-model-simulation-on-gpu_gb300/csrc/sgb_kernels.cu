@@ -781,10 +781,23 @@ __device__ __forceinline__ void step_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-__global__ void k_chunk_begin(StepArgs a) {
-  a.ctl->t_rel = 0;
-  a.ctl->raster_count = 0;
-  a.raster_off[0] = 0;
+// Start of a chunk of `steps` steps: clears its counts and, for a persistent
+// launch, the barrier counter and the board (n_bar words), and takes new
+// stimulus sources from the host's pinned copy.
+__global__ void __launch_bounds__(kBlock) k_chunk_begin(StepArgs a, uint32_t steps, uint32_t n_bar,
+                                                        const SrcDev* srcs) {
+  const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x, n = gridDim.x * kBlock;
+  for (size_t j = gtid; j < (size_t)steps * a.n_segs; j += n) a.counts[j] = 0u;
+  for (uint32_t j = gtid; j < n_bar; j += n) reinterpret_cast<uint32_t*>(a.bar)[j] = 0u;
+  if (srcs)
+    for (uint32_t j = gtid; j < a.n_srcs * (uint32_t)(sizeof(SrcDev) / 8); j += n)
+      reinterpret_cast<unsigned long long*>(const_cast<SrcDev*>(a.srcs))[j] =
+          reinterpret_cast<const volatile unsigned long long*>(srcs)[j];
+  if (gtid == 0) {
+    a.ctl->t_rel = 0;
+    a.ctl->raster_count = 0;
+    a.raster_off[0] = 0;
+  }
 }
 
 __global__ void __launch_bounds__(kBlock) k_update(StepArgs a) {
@@ -1175,10 +1188,17 @@ __global__ void __launch_bounds__(kBlock) k_plast_reset(StepArgs a) {
   }
 }
 
-// Per-segment spike totals of the chunk, folded into the FP64 accumulators.
-__global__ void __launch_bounds__(kBlock) k_chunk_end(StepArgs a) {
+// Per-segment spike totals of the chunk, folded into the FP64 accumulators;
+// the error flags and, when the host wants them and they are few, the chunk's
+// counts go to pinned host memory from here, without a copy of their own.
+__global__ void __launch_bounds__(kBlock) k_chunk_end(StepArgs a, uint32_t* host_err, uint32_t* host_counts) {
   const uint32_t seg = blockIdx.x;
   const uint32_t steps = a.ctl->t_rel;
+  if (host_counts)
+    for (uint32_t j = seg * kBlock + threadIdx.x; j < steps * a.n_segs; j += gridDim.x * kBlock)
+      host_counts[j] = a.counts[j];
+  if (seg == 0 && threadIdx.x == 0) *host_err = a.ctl->error;
+  if (seg >= a.n_segs) return;
   unsigned long long s = 0;
   for (uint32_t r = threadIdx.x; r < steps; r += blockDim.x) s += a.counts[(size_t)r * a.n_segs + seg];
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(kFull, s, o);
@@ -2681,8 +2701,10 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
 
 }  // namespace
 
-cudaError_t launch_chunk_begin(const StepArgs& a, cudaStream_t s) {
-  k_chunk_begin<<<1, 1, 0, s>>>(a);
+cudaError_t launch_chunk_begin(const StepArgs& a, uint32_t steps, uint32_t n_bar, const SrcDev* srcs,
+                               cudaStream_t s) {
+  const size_t n = std::max<size_t>((size_t)steps * a.n_segs, n_bar);
+  k_chunk_begin<<<(int)std::min<size_t>(n / (4 * kBlock) + 1, 152), kBlock, 0, s>>>(a, steps, n_bar, srcs);
   return cudaGetLastError();
 }
 
@@ -2806,9 +2828,8 @@ int pull_blocks_per_sm(const StepArgs& a) {
   return n > 0 ? n : 1;
 }
 
-cudaError_t launch_chunk_end(const StepArgs& a, cudaStream_t s) {
-  if (!a.n_segs) return cudaSuccess;
-  k_chunk_end<<<a.n_segs, kBlock, 0, s>>>(a);
+cudaError_t launch_chunk_end(const StepArgs& a, uint32_t* host_err, uint32_t* host_counts, cudaStream_t s) {
+  k_chunk_end<<<std::max(a.n_segs, 1u), kBlock, 0, s>>>(a, host_err, host_counts);
   return cudaGetLastError();
 }
 
