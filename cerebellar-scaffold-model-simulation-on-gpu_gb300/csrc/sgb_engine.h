@@ -71,6 +71,11 @@ struct Sim {
   void* d_plast = nullptr;
   void* d_heavy = nullptr;    // fused kernel's heavy words: split points, index, lists
   size_t heavy_bytes = 0;
+  // sim_get_state: the states in id order, in pinned or device memory, and
+  // each segment's first id.
+  int64_t n_state = 0;
+  void *h_state = nullptr, *d_state = nullptr;
+  long long* first_ids = nullptr;
   void* d_sorted = nullptr;   // dense tables in the one-barrier resident kernel's form
   size_t sorted_bytes = 0;
   size_t off_recent = 0;      // per-cell spike registers inside d_plast

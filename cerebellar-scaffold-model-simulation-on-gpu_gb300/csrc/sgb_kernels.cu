@@ -1212,6 +1212,26 @@ __global__ void __launch_bounds__(kBlock) k_chunk_end(StepArgs a, uint32_t* host
   }
 }
 
+// Cell states in id order (first[seg]: a segment's first id), as the host
+// reads them: potential, two conductances, refractory steps.  One thread per
+// padded cell; bound by the copy of its output to the host.
+__global__ void __launch_bounds__(kBlock) k_state_out(StepArgs a, const long long* first, float* u, float2* g,
+                                                      int32_t* ref) {
+  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= a.n_pad) return;
+  const uint32_t seg = a.seg_of_word[i >> 5];
+  if (seg == 0xFFFFu) return;
+  const SegDev& sd = a.segs[seg];
+  const uint32_t local = i - sd.base;
+  if (local >= sd.count) return;
+  const long long o = first[seg] + local;
+  const float x = a.su[i];
+  const int32_t r = sd.kind == kSegLif ? unpack_ref(x) : 0;
+  u[o] = r ? sd.Vr : x;
+  g[o] = a.sg[i];
+  ref[o] = r;
+}
+
 // ---- persistent driver ----------------------------------------------------------
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
   unsigned long long v;
@@ -2705,6 +2725,12 @@ cudaError_t launch_chunk_begin(const StepArgs& a, uint32_t steps, uint32_t n_bar
                                cudaStream_t s) {
   const size_t n = std::max<size_t>((size_t)steps * a.n_segs, n_bar);
   k_chunk_begin<<<(int)std::min<size_t>(n / (4 * kBlock) + 1, 152), kBlock, 0, s>>>(a, steps, n_bar, srcs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_state_out(const StepArgs& a, const long long* first, float* u, float2* g, int32_t* ref,
+                             cudaStream_t s) {
+  k_state_out<<<(a.n_pad + kBlock - 1) / kBlock, kBlock, 0, s>>>(a, first, u, g, ref);
   return cudaGetLastError();
 }
 
