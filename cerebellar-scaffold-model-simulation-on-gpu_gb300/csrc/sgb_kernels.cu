@@ -3007,6 +3007,8 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
   const size_t smem = fused ? a.row_smem
                      : (a.seg_smem ? seg_smem_bytes(a) : 0) +
                            ((a.n_pull_units && a.pull_sum) ? pull_sum_bytes(a) : 0);
+  // Heavy words without the shared memory that the kernel addresses for them.
+  if (fused && a.hv_words && a.row_smem < fused_heavy_bytes(a, blocks)) return cudaErrorInvalidValue;
   const uint32_t threads = fused ? fused_threads(a, blocks) : kPersistBlock;
   return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads), params, smem, s);
 }
