@@ -1729,8 +1729,8 @@ __device__ __forceinline__ uint2 stdp_sub(const StepArgs& a, uint32_t x, uint32_
 // sees them): threads screen sub-units, then warps update those that can
 // change.  s_sub: the held sub-units' stdp_sub, or NULL.  Run by the block's
 // first n_thr threads, which meet on block barrier 1 (0 when all run it);
-// it ends with that barrier when anything was updated.  s_n[2] counts the
-// active sub-units of alternate rounds, par the next round's.
+// every round but a last one without updates ends with that barrier.  s_n[2]
+// counts the active sub-units of alternate rounds, par the next round's.
 template <bool BF16, bool EARLY>
 __device__ __forceinline__ void stdp_own(const StepArgs& a, const HistRows& h,
                                          const unsigned long long* recent, const uint2* s_sub,
@@ -1751,14 +1751,16 @@ __device__ __forceinline__ void stdp_own(const StepArgs& a, const HistRows& h,
     }
     sync();
     const uint32_t n = s_n[par];
-    if (threadIdx.x == 0) s_n[par ^ 1u] = 0;  // its readers were before this barrier
+    // The next round's count.  Its readers were before this barrier; its next
+    // writers come after the one that ends the round.
+    if (threadIdx.x == 0) s_n[par ^ 1u] = 0;
     for (uint32_t j = threadIdx.x >> 5; j < n; j += n_thr >> 5) {
       const uint32_t v = s_list[j];
       uint32_t k, o0;
       stdp_sub(a, b + (v & 0xFFFFu), &k, &o0);
       stdp_unit<BF16, true, EARLY>(a, PullUnit{k, o0}, h, pad, recent, v >> 31);
     }
-    if (n) sync();
+    if (n || b + n_thr < n_sub) sync();
   }
 }
 
