@@ -1139,9 +1139,13 @@ int sim_set_rates(Sim& s, int32_t net, int32_t n, const float* rates) {
       if (int rc = wait_stream(s)) return rc;
     memcpy(s.h_srcs, s.srcs.data(), s.srcs.size() * sizeof(SrcDev));
     s.srcs_dirty = true;
-    // The caller's stream may be capturing the steps, or replaying captured
-    // ones, which must find the new sources in place.
-    if (shared) return upload_sources(s);
+    // Steps that the caller captured on a stream of its own may be replayed at
+    // any time from now on, also while the handle is back on its own stream,
+    // and must find the new sources in place.
+    if (s.lent) {
+      if (int rc = upload_sources(s)) return rc;
+      if (!shared) return wait_stream(s);
+    }
   }
   return SGB_OK;
 }
@@ -1303,6 +1307,7 @@ int sim_set_stream(Sim& s, cudaStream_t st) {
     SGB_CUDA(l2_window_on(s, next, true));
   }
   s.stream = next;
+  s.lent = s.lent || st;
   for (auto& kv : s.graphs) cudaGraphExecDestroy(kv.second);
   s.graphs.clear();
   return SGB_OK;

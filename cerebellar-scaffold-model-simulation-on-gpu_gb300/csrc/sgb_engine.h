@@ -91,6 +91,7 @@ struct Sim {
   SrcDev* h_srcs = nullptr;  // pinned staging of the source table
   bool srcs_dirty = false;   // h_srcs not yet on the device: the next chunk takes it along
   bool busy = false;         // work that may read h_srcs has been issued since the last wait
+  bool lent = false;         // has been on a stream of the caller's, who may have captured steps there
   uint32_t* h_err = nullptr; // pinned: the device's error flags at the end of the last chunk
 
   // Host staging for outputs.
