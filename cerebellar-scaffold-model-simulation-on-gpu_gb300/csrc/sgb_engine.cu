@@ -1016,6 +1016,12 @@ static int take_device_error(Sim& s, uint32_t* bits) {
   return SGB_OK;
 }
 
+// After the device's control block was replaced: the flags to report are its own.
+static int reload_device_error(Sim& s) {
+  SGB_CUDA(cudaMemcpy(s.h_err, &s.args.ctl->error, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  return SGB_OK;
+}
+
 int sim_enqueue(Sim& s, int64_t n_steps) {
   if (n_steps < 0) return set_error(SGB_ERR_ARG, "n_steps is negative");
   for (int64_t done = 0; done < n_steps;) {
@@ -1562,6 +1568,7 @@ int sim_autotune(Sim& s, int32_t n_steps, const char* cache_path) {
     shape = cur;
   }
   if (save(true)) return fail(set_error(SGB_ERR_CUDA, "autotune restore failed"));
+  if ((rc = reload_device_error(s))) return fail(rc);
   // The restored state carries the deliveries in flight under the modes the
   // handle had before tuning.
   if ((rc = handover_modes(s, modes0))) return fail(rc);
@@ -1770,6 +1777,7 @@ int sim_checkpoint(Sim& s, void* buf, int64_t size, bool load) {
       s.srcs_dirty = false;
       SGB_CUDA(cudaMemcpy((void*)s.args.srcs, s.h_srcs, nsrc, cudaMemcpyHostToDevice));
     }
+    return reload_device_error(s);
   } else if (nsrc) {
     memcpy(p, s.srcs.data(), nsrc);
   }
