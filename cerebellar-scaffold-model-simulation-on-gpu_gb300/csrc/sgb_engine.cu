@@ -282,6 +282,14 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   return SGB_OK;
 }
 
+// A copy from pageable host memory may return before its data have reached the
+// device, and the handle's stream does not wait for the stream that makes such
+// copies: this does, before anything that reads them is launched.
+static int wait_copies() {
+  SGB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return SGB_OK;
+}
+
 // Rebuilds the merged push table (every projection in CSR mode, cell-major)
 // and the dense-pull work lists, uploads them, and drops captured graphs.
 static int upload_modes(Sim& s) {
@@ -356,6 +364,7 @@ static int upload_modes(Sim& s) {
     }
     a.pull_info = (const uint4*)s.d_sorted;
     a.pull_sorted = (const uint32_t*)((char*)s.d_sorted + (size_t)a.n_pull_units * sizeof(uint4));
+    if (int rc = wait_copies()) return rc;
     SGB_CUDA(launch_pull_sort(a, s.stream));
   }
   const bool fused = total > 0 && s.persistent_blocks > 0 &&
@@ -383,7 +392,7 @@ static int upload_modes(Sim& s) {
   }
   for (auto& kv : s.graphs) cudaGraphExecDestroy(kv.second);
   s.graphs.clear();
-  return SGB_OK;
+  return wait_copies();
 }
 
 int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seeds, int32_t n,
@@ -1280,7 +1289,7 @@ static int handover_modes(Sim& s, const std::vector<uint32_t>& before) {
     SGB_CUDA(cudaMemcpy((int2*)s.args.ring + (size_t)slot_of(j) * s.n_pad,
                         slots.data() + (size_t)(j - 1) * s.n_pad, (size_t)s.n_pad * 8,
                         cudaMemcpyHostToDevice));
-  return SGB_OK;
+  return wait_copies();
 }
 
 static std::vector<uint32_t> current_modes(const Sim& s) {
@@ -1777,6 +1786,7 @@ int sim_checkpoint(Sim& s, void* buf, int64_t size, bool load) {
       s.srcs_dirty = false;
       SGB_CUDA(cudaMemcpy((void*)s.args.srcs, s.h_srcs, nsrc, cudaMemcpyHostToDevice));
     }
+    if (int rc = wait_copies()) return rc;
     return reload_device_error(s);
   } else if (nsrc) {
     memcpy(p, s.srcs.data(), nsrc);
