@@ -245,10 +245,8 @@ cudaError_t launch_state_out(const StepArgs& a, const long long* first, float* u
 cudaError_t launch_chunk_end(const StepArgs& a, uint32_t* host_err, uint32_t* host_counts, cudaStream_t s);
 // One cooperative launch advancing n_steps; grid = blocks (all co-resident).
 cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, cudaStream_t s);
-// Largest dynamic shared memory the fused persistent kernel can take for push
-// rows, and setting it (both weight types) before launches that use it.
+// Largest dynamic shared memory that every form of the fused persistent kernel can take.
 uint32_t fused_row_smem_max();
-cudaError_t set_fused_row_smem(uint32_t bytes);
 int persistent_blocks_per_sm(bool bf16);
 // Shared memory that the fused kernel's heavy words (a.hv_*) take on a grid of `blocks`.
 size_t fused_heavy_bytes(const StepArgs& a, int blocks);

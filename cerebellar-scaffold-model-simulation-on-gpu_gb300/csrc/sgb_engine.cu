@@ -385,10 +385,7 @@ static int upload_modes(Sim& s) {
     const uint64_t bytes = std::min<uint64_t>((most + 255) & ~255ull, fused_row_smem_max());
     // Own rows alone are worth the shared memory from 1 KiB on; heavy words
     // keep their delay line and synapses there however small they are.
-    if (bytes >= 1024 || a.hv_words) {
-      SGB_CUDA(set_fused_row_smem((uint32_t)bytes));
-      a.row_smem = (uint32_t)bytes;
-    }
+    if (bytes >= 1024 || a.hv_words) a.row_smem = (uint32_t)bytes;
   }
   for (auto& kv : s.graphs) cudaGraphExecDestroy(kv.second);
   s.graphs.clear();

@@ -2841,6 +2841,15 @@ static size_t dyn_smem_max(const void* fn) {
   return ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)255;
 }
 
+// The fused kernel's forms: [BF16][timeline][words per warp - 1].
+#define SGB_FUSED_FORMS(B)                                                      \
+  (const void*)k_persistent_fused<B, 0, 1>, (const void*)k_persistent_fused<B, 0, 2>,     \
+      (const void*)k_persistent_fused<B, 1, 1>, (const void*)k_persistent_fused<B, 1, 2>, \
+      (const void*)k_persistent_fused<B, 2, 1>, (const void*)k_persistent_fused<B, 2, 2>
+constexpr uint32_t kFusedForms = 6;
+static const void* const kFusedKernels[] = {SGB_FUSED_FORMS(false), SGB_FUSED_FORMS(true)};
+#undef SGB_FUSED_FORMS
+
 cudaError_t pull_setup() {
   const int mx = (int)kPullSumMax;
   cudaError_t e;
@@ -2860,6 +2869,11 @@ cudaError_t pull_setup() {
   if ((e = cudaFuncSetAttribute(k_persistent<false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))) return e;
   if ((e = cudaFuncSetAttribute(k_persistent_resident<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx)))
     return e;
+  // The limit belongs to the function, for every handle of the process, so it
+  // is the most that the function can take; a launch names its own size.
+  for (const void* fn : kFusedKernels)
+    if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem_max(fn))))
+      return e;
   for (const void* fn : kPullKernels)
     if ((e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn_smem_max(fn))))
       return e;
@@ -2876,15 +2890,6 @@ cudaError_t launch_chunk_end(const StepArgs& a, uint32_t* host_err, uint32_t* ho
   k_chunk_end<<<std::max(a.n_segs, 1u), kBlock, 0, s>>>(a, host_err, host_counts);
   return cudaGetLastError();
 }
-
-// The fused kernel's forms: [BF16][timeline][words per warp - 1].
-#define SGB_FUSED_FORMS(B)                                                      \
-  (const void*)k_persistent_fused<B, 0, 1>, (const void*)k_persistent_fused<B, 0, 2>,     \
-      (const void*)k_persistent_fused<B, 1, 1>, (const void*)k_persistent_fused<B, 1, 2>, \
-      (const void*)k_persistent_fused<B, 2, 1>, (const void*)k_persistent_fused<B, 2, 2>
-constexpr uint32_t kFusedForms = 6;
-static const void* const kFusedKernels[] = {SGB_FUSED_FORMS(false), SGB_FUSED_FORMS(true)};
-#undef SGB_FUSED_FORMS
 
 // Words per block, at most, and per warp: a warp without a word still runs a
 // step's bookkeeping, and in steps bound by latency those instructions delay
@@ -3019,15 +3024,6 @@ uint32_t fused_row_smem_max() {
   size_t most = ~(size_t)0;
   for (const void* fn : kFusedKernels) most = std::min(most, dyn_smem_max(fn));
   return (uint32_t)most;
-}
-
-cudaError_t set_fused_row_smem(uint32_t bytes) {
-  for (const void* fn : kFusedKernels) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e) return e;
-  }
-  return cudaSuccess;
 }
 
 }  // namespace sgb
