@@ -195,6 +195,29 @@ static bool build_ell(const Projection& pr, int32_t npost, uint32_t pre_base, ui
   return true;
 }
 
+// Room for `need` bytes of derived tables, kept from one call for the next.
+// *ok says whether there is; without memory for them their kernel's general
+// form runs, which needs none.
+static int grow_tables(Sim& s, void** p, size_t* have, size_t need, bool* ok) {
+  *ok = true;
+  if (need <= *have) return SGB_OK;
+  if (*p) cudaFree(*p);
+  *p = nullptr;
+  s.push_bytes -= *have;
+  *have = 0;
+  const cudaError_t e = cudaMalloc(p, need);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    *p = nullptr;
+    *ok = false;
+    return SGB_OK;
+  }
+  SGB_CUDA(e);
+  *have = need;
+  s.push_bytes += need;
+  return SGB_OK;
+}
+
 // The fused kernel's heavy words: 32-cell words with a row of at least
 // kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
 // block has room for the words' synapses onto its cells (half of its shared
@@ -260,14 +283,13 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   }
   const size_t o_idx = align_up((size_t)s.n_pad * 4, 256), o_off = align_up(o_idx + index.size() * 2, 256);
   const size_t o_syn = align_up(o_off + off.size() * 2, 256), need = o_syn + list.size() * sizeof(uint2);
-  if (need > s.heavy_bytes) {
-    if (s.d_heavy) cudaFree(s.d_heavy);
-    s.d_heavy = nullptr;
-    s.push_bytes -= s.heavy_bytes;
-    s.heavy_bytes = 0;
-    SGB_CUDA(cudaMalloc(&s.d_heavy, need));
-    s.heavy_bytes = need;
-    s.push_bytes += need;
+  bool ok;
+  if (int rc = grow_tables(s, &s.d_heavy, &s.heavy_bytes, need, &ok)) return rc;
+  if (!ok) {  // every row stays with its cell's block
+    a.hv_words = a.hv_cap = 0;
+    s.n_heavy_cells = 0;
+    own_end.assign(row.begin() + 1, row.end());
+    return SGB_OK;
   }
   char* hb = (char*)s.d_heavy;
   SGB_CUDA(cudaMemcpy(hb, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
@@ -353,15 +375,11 @@ static int upload_modes(Sim& s) {
   if (a.pull_smem) {
     // Its entries, sorted per unit: 4 B each and 16 B per unit, on the device.
     const size_t need = (size_t)a.n_pull_units * (kPullUnit * 4 + sizeof(uint4));
-    if (need > s.sorted_bytes) {
-      if (s.d_sorted) cudaFree(s.d_sorted);
-      s.d_sorted = nullptr;
-      s.push_bytes -= s.sorted_bytes;
-      s.sorted_bytes = 0;
-      SGB_CUDA(cudaMalloc(&s.d_sorted, need));
-      s.sorted_bytes = need;
-      s.push_bytes += need;
-    }
+    bool ok;
+    if (int rc = grow_tables(s, &s.d_sorted, &s.sorted_bytes, need, &ok)) return rc;
+    if (!ok) a.pull_smem = a.pull_held = 0;  // the two-barrier form
+  }
+  if (a.pull_smem) {
     a.pull_info = (const uint4*)s.d_sorted;
     a.pull_sorted = (const uint32_t*)((char*)s.d_sorted + (size_t)a.n_pull_units * sizeof(uint4));
     if (int rc = wait_copies()) return rc;
