@@ -195,26 +195,24 @@ static bool build_ell(const Projection& pr, int32_t npost, uint32_t pre_base, ui
   return true;
 }
 
-// Room for `need` bytes of derived tables, kept from one call for the next.
-// *ok says whether there is; without memory for them their kernel's general
-// form runs, which needs none.
-static int grow_tables(Sim& s, void** p, size_t* have, size_t need, bool* ok) {
-  *ok = true;
-  if (need <= *have) return SGB_OK;
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  s.push_bytes -= *have;
-  *have = 0;
-  const cudaError_t e = cudaMalloc(p, need);
+// Memory for derived tables, taken once, at the size they can have at most
+// (*ok: there is any; without it their kernel's general form runs, which needs
+// none).  Steps that the caller captured keep the addresses and sizes of their
+// tables: a replay after a mode change must find them there, and one after the
+// modes are back as they were finds the same contents.  So tables never move,
+// and their parts keep their places.
+static int derived_tables(Sim& s, void** p, size_t bytes, bool* ok) {
+  *ok = *p != nullptr;
+  if (*ok) return SGB_OK;
+  const cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     *p = nullptr;
-    *ok = false;
     return SGB_OK;
   }
   SGB_CUDA(e);
-  *have = need;
-  s.push_bytes += need;
+  *ok = true;
+  s.push_bytes += bytes;
   return SGB_OK;
 }
 
@@ -222,7 +220,8 @@ static int grow_tables(Sim& s, void** p, size_t* have, size_t need, bool* ok) {
 // kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
 // block has room for the words' synapses onto its cells (half of its shared
 // memory with the delay line; the push rows get the rest).  Fills the handle's
-// tables and takes the words' rows out of own_end (what a cell's block pushes).
+// tables and takes the words' rows out of own_end (the end of what a cell's
+// block pushes; the caller uploads it to the tables' start).
 static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
                         const std::vector<uint32_t>& syn, const std::vector<float>& wf,
                         const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
@@ -282,9 +281,10 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
     }
   }
   const size_t o_idx = align_up((size_t)s.n_pad * 4, 256), o_off = align_up(o_idx + index.size() * 2, 256);
-  const size_t o_syn = align_up(o_off + off.size() * 2, 256), need = o_syn + list.size() * sizeof(uint2);
+  const size_t o_syn = align_up(o_off + (size_t)B * (kHeavyWords * 32u + 1u) * 2, 256);
+  const size_t most_cap = std::min<size_t>(budget / sizeof(uint2), (size_t)std::max<int64_t>(s.n_syn, 1));
   bool ok;
-  if (int rc = grow_tables(s, &s.d_heavy, &s.heavy_bytes, need, &ok)) return rc;
+  if (int rc = derived_tables(s, &s.d_heavy, o_syn + B * most_cap * sizeof(uint2), &ok)) return rc;
   if (!ok) {  // every row stays with its cell's block
     a.hv_words = a.hv_cap = 0;
     s.n_heavy_cells = 0;
@@ -292,7 +292,6 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
     return SGB_OK;
   }
   char* hb = (char*)s.d_heavy;
-  SGB_CUDA(cudaMemcpy(hb, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
   SGB_CUDA(cudaMemcpy(hb + o_idx, index.data(), index.size() * 2, cudaMemcpyHostToDevice));
   SGB_CUDA(cudaMemcpy(hb + o_off, off.data(), off.size() * 2, cudaMemcpyHostToDevice));
   SGB_CUDA(cudaMemcpy(hb + o_syn, list.data(), list.size() * sizeof(uint2), cudaMemcpyHostToDevice));
@@ -374,14 +373,13 @@ static int upload_modes(Sim& s) {
   plan_persistent_pull(a, s.persistent_blocks);
   if (a.pull_smem) {
     // Its entries, sorted per unit: 4 B each and 16 B per unit, on the device.
-    const size_t need = (size_t)a.n_pull_units * (kPullUnit * 4 + sizeof(uint4));
     bool ok;
-    if (int rc = grow_tables(s, &s.d_sorted, &s.sorted_bytes, need, &ok)) return rc;
+    if (int rc = derived_tables(s, &s.d_sorted, s.cap_units * (kPullUnit * 4 + sizeof(uint4)), &ok)) return rc;
     if (!ok) a.pull_smem = a.pull_held = 0;  // the two-barrier form
   }
   if (a.pull_smem) {
-    a.pull_info = (const uint4*)s.d_sorted;
-    a.pull_sorted = (const uint32_t*)((char*)s.d_sorted + (size_t)a.n_pull_units * sizeof(uint4));
+    a.pull_sorted = (const uint32_t*)s.d_sorted;
+    a.pull_info = (const uint4*)((char*)s.d_sorted + s.cap_units * kPullUnit * 4);
     if (int rc = wait_copies()) return rc;
     SGB_CUDA(launch_pull_sort(a, s.stream));
   }
@@ -390,6 +388,9 @@ static int upload_modes(Sim& s) {
   a.row_smem = 0;
   std::vector<uint32_t> own_end(row.begin() + 1, row.end());
   if (int rc = upload_heavy(s, fused, row, syn, wf, wh, own_end)) return rc;
+  // The ends go with the rows also without heavy words (captured steps).
+  if (s.d_heavy)
+    SGB_CUDA(cudaMemcpy(s.d_heavy, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
   if (fused) {
     // Shared memory for the push rows of the block holding the most synapses
     // (word slot ws runs in block ws mod blocks), beside the heavy words'.
@@ -623,8 +624,7 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
       upd_words.push_back(w);
     }
   }
-  size_t cap_units = 0;
-  for (const ProjDev& P : s.projs) cap_units += (P.ell_n + kPullUnit - 1) / kPullUnit;
+  for (const ProjDev& P : s.projs) s.cap_units += (P.ell_n + kPullUnit - 1) / kPullUnit;
 
   // ---- device memory ---------------------------------------------------------
   s.ell_bytes = std::max<size_t>(pool, 256);
@@ -668,7 +668,7 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   const size_t o_mask = take((size_t)s.n_pad * 4);
   const size_t o_outdeg = take((size_t)s.n_pad * 4);
   const size_t o_words = take(std::max<size_t>(upd_words.size(), 1) * 4);
-  const size_t o_units = take(std::max<size_t>(cap_units, 1) * sizeof(PullUnit));
+  const size_t o_units = take(std::max<size_t>(s.cap_units, 1) * sizeof(PullUnit));
   const size_t o_su = take((size_t)s.n_pad * sizeof(float));
   const size_t o_sg = take((size_t)s.n_pad * sizeof(float2));
   const size_t o_ring = take((size_t)s.ring_slots * s.n_pad * 8);

@@ -58,6 +58,7 @@ struct Sim {
   size_t ell_bytes = 0;
   void* d_push = nullptr;   // merged push table (capacity: every synapse)
   size_t push_bytes = 0;
+  size_t cap_units = 0;     // dense-pull units with every projection dense
   void* d_misc = nullptr;   // state, ring, history, lists, descriptors
   size_t misc_bytes = 0;
   StepArgs args{};
@@ -70,14 +71,12 @@ struct Sim {
   // Plasticity (STDP) of plastic projections.
   void* d_plast = nullptr;
   void* d_heavy = nullptr;    // fused kernel's heavy words: split points, index, lists
-  size_t heavy_bytes = 0;
   // sim_get_state: the states in id order, in pinned or device memory, and
   // each segment's first id.
   int64_t n_state = 0;
   void *h_state = nullptr, *d_state = nullptr;
   long long* first_ids = nullptr;
   void* d_sorted = nullptr;   // dense tables in the one-barrier resident kernel's form
-  size_t sorted_bytes = 0;
   size_t off_recent = 0;      // per-cell spike registers inside d_plast
   std::vector<PlastHost> plast;
   // Per-step drivers with early plasticity rules: k_stdp runs on `side`,

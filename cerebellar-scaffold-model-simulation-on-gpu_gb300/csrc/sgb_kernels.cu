@@ -2233,8 +2233,10 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
     for (uint32_t j = threadIdx.x; j < n_line * n_cell; j += n_thr) s_line[j] = make_int2(0, 0);
     const uint32_t n_off = a.hv_words * 32u + 1u;
     const uint16_t* off = a.hv_off + (size_t)blockIdx.x * n_off;
-    for (uint32_t j = threadIdx.x; j < n_off; j += n_thr) s_hoff[j] = __ldg(off + j);
-    const uint32_t n = __ldg(off + n_off - 1u);
+    // Within this launch's list also when the caller replays captured steps
+    // whose tables have changed since.
+    const uint32_t n = min((uint32_t)__ldg(off + n_off - 1u), a.hv_cap);
+    for (uint32_t j = threadIdx.x; j < n_off; j += n_thr) s_hoff[j] = (uint16_t)min((uint32_t)__ldg(off + j), n);
     const uint2* src = a.hv_syn + (size_t)blockIdx.x * a.hv_cap;
     for (uint32_t j = threadIdx.x; j < n; j += n_thr) s_hsyn[j] = __ldg(src + j);
   }
