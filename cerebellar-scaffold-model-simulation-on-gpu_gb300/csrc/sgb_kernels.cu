@@ -859,8 +859,11 @@ __global__ void __launch_bounds__(kBlock) k_deliver(StepArgs a) {
 // loads its 32 entries of a unit at once, settles every entry whose summary
 // bit is clear in shared memory, and walks the few that passed four at a
 // time (usually one trip per warp), loading each entry again (an L1 hit) and
-// then its history word (through L1: the history is read-only in this
-// launch).  Without room for the summary (SUM false) every entry walks.
+// then its history word (an ordinary load, through L1: as a programmatic
+// dependent this grid may be resident while k_update still writes the step's
+// row, which the read-only path rules out and step_begin's wait orders; loaded
+// at L2 instead, 1,388,250 cells take 59 us per step, not 53).  Without room
+// for the summary (SUM false) every entry walks.
 template <bool BF16, bool SUM>
 __global__ void __launch_bounds__(kPullBlock, 1) k_pull(StepArgs a) {
   constexpr uint32_t E = kPullUnit / 32;  // entries per lane per unit
@@ -916,7 +919,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) k_pull(StepArgs a) {
       for (uint32_t j = 0; j < W; ++j) ev[j] = ks[j] < E ? __ldg(src + ks[j] * 32u) : 0u;
 #pragma unroll
       for (uint32_t j = 0; j < W; ++j)
-        hw[j] = ks[j] < E ? __ldg(hb + (ev[j] >> 5)) : 0u;
+        hw[j] = ks[j] < E ? hb[ev[j] >> 5] : 0u;
 #pragma unroll
       for (uint32_t j = 0; j < W; ++j) {
         if (ks[j] < E && ((hw[j] >> (ev[j] & 31u)) & 1u)) {
@@ -988,7 +991,7 @@ __global__ void __launch_bounds__(kPullBlock, 1) k_pull_vec(StepArgs a) {
       for (uint32_t j = 0; j < W; ++j)
         ev[j] = ms[j] < E ? __ldg(base + (ms[j] >> 2) * 128u + (ms[j] & 3u)) : 0u;
 #pragma unroll
-      for (uint32_t j = 0; j < W; ++j) hw[j] = ms[j] < E ? __ldg(hb + (ev[j] >> 5)) : 0u;
+      for (uint32_t j = 0; j < W; ++j) hw[j] = ms[j] < E ? hb[ev[j] >> 5] : 0u;
 #pragma unroll
       for (uint32_t j = 0; j < W; ++j) {
         if (ms[j] < E && ((hw[j] >> (ev[j] & 31u)) & 1u)) {
