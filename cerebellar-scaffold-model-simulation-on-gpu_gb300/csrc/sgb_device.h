@@ -228,6 +228,7 @@ struct StepArgs {
   unsigned long long* board;      // [4][kHeavyWords] {step tag, spike bits}, zeroed per launch, after bar
   int32_t bf16;
   int32_t substeps;
+  uint32_t sms;                   // the device's SMs
 };
 
 // Launch wrappers (sgb_kernels.cu).  All return the launch status.

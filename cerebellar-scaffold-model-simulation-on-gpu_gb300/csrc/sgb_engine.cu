@@ -741,6 +741,7 @@ int sim_create(const sgb_config& cfg, sgb_net* const* nets, const uint64_t* seed
   a.raster_cap = s.raster_cap;
   a.bf16 = s.bf16 ? 1 : 0;
   a.substeps = cfg.substeps;
+  a.sms = (uint32_t)s.sm_count;
   a.bar_extra = (uint32_t)cfg.barrier_test_extra;
   s.deliver_blocks = 2 * s.sm_count;
   a.item_log2 = 7;  // fused kernel's late-push timelines: push items of 128 synapses (or 64)

@@ -2740,7 +2740,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
 cudaError_t launch_chunk_begin(const StepArgs& a, uint32_t steps, uint32_t n_bar, const SrcDev* srcs,
                                cudaStream_t s) {
   const size_t n = std::max<size_t>((size_t)steps * a.n_segs, n_bar);
-  k_chunk_begin<<<(int)std::min<size_t>(n / (4 * kBlock) + 1, 152), kBlock, 0, s>>>(a, steps, n_bar, srcs);
+  k_chunk_begin<<<(int)std::min<size_t>(n / (4 * kBlock) + 1, a.sms), kBlock, 0, s>>>(a, steps, n_bar, srcs);
   return cudaGetLastError();
 }
 
@@ -2773,7 +2773,7 @@ cudaError_t launch_update(const StepArgs& a, cudaStream_t s) {
   // The loop's warps get their words ahead, so words that differ much in work
   // (input cells draw for each substep) are better left to waves of blocks:
   // 370,200 cells, ten substeps, 14.4 us per step in waves, 16.4 looped.
-  const uint32_t blocks = (a.n_words + kBlock / 32 - 1) / (kBlock / 32), most = 152u * kUpdateBlocks;
+  const uint32_t blocks = (a.n_words + kBlock / 32 - 1) / (kBlock / 32), most = a.sms * kUpdateBlocks;
   const bool loop = blocks > most && a.substeps == 1;
   return step_launch(loop ? k_update<true> : k_update<false>, a, loop ? most : blocks, kBlock, 0, s);
 }
