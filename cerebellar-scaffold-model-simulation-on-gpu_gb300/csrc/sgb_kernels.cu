@@ -777,14 +777,16 @@ __device__ __forceinline__ void ix_advance(const StepArgs& a, StepIdx& ix) {
 // ---- per-step kernels (CUDA-graph driver) ----------------------------------
 // A step's kernels depend on one another, but their launches need not: each is
 // launched as a programmatic dependent of the one before (step_launch), so its
-// blocks are scheduled while that one still runs, and waits here before its
+// blocks are scheduled while that one still runs, and waits (step_wait) before its
 // first access for that kernel to end and its writes to be visible.  Every
 // block passes this point, so a kernel's end implies the end of all before it.
 // In a graph: 92,550 cells event-driven 6.85 -> 6.5 us per step, every
 // projection dense 13.3 -> 12.2, 9,255 cells 5.8 -> 5.4.
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void step_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void step_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  step_wait();
+  step_next();
 }
 
 // Start of a chunk of `steps` steps: clears its counts and, for a persistent
@@ -811,10 +813,17 @@ __global__ void __launch_bounds__(kBlock) k_chunk_begin(StepArgs a, uint32_t ste
 // once, not in every wave of blocks (per step: 370,200 cells 10.3 -> 9.3 us,
 // 925,500 15.5 -> 13.2, 1,388,250 dense 56.8 -> 51.2; 3 blocks per SM 14.2 and
 // 53, 5 14.3 and 52.7).
+//   A grid of more than kUpdateBlocks per SM lets the next kernel start only as
+// its blocks end: started before, the delivery's blocks crowd onto the SMs that
+// have room first (300,000 cells in ten substeps, 150 Hz input: 33.2 us per step,
+// 28.8 so; scaffolds of 370,200 cells 14.4 and 14.2; smaller grids leave room on
+// every SM, and start it at once: 92,550 cells in two substeps 7.9, else 8.0).
 constexpr uint32_t kUpdateBlocks = 4;  // per SM
 template <bool LOOP>
 __global__ void __launch_bounds__(kBlock, LOOP ? kUpdateBlocks : 0) k_update(StepArgs a) {
-  step_begin();
+  step_wait();
+  const bool early = LOOP || gridDim.x <= a.sms * kUpdateBlocks;
+  if (early) step_next();
   const uint32_t gtid = blockIdx.x * kBlock + threadIdx.x;
   const uint32_t w = gtid >> 5;
   const StepIdx ix = step_of(a);
@@ -823,6 +832,7 @@ __global__ void __launch_bounds__(kBlock, LOOP ? kUpdateBlocks : 0) k_update(Ste
     update_words<true, false, false, false>(a, w, gridDim.x * (kBlock / 32), ix, {nullptr, nullptr});
   else if (w < a.n_words)
     update_word(a, w, ix);
+  if (!early) step_next();
 }
 
 // Delivery of step t; the last block to finish also advances the step
