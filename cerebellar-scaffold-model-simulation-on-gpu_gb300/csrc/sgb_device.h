@@ -49,6 +49,11 @@ constexpr uint32_t kPushChunk = 256;  // synapses per push work item (8 per lane
 constexpr uint32_t kHeavyMin = 128;
 constexpr uint32_t kHeavyMinSub = 256;
 constexpr uint32_t kHeavyWords = 128;
+// Spikes a step that the stimulus is expected to cause in heavy words, up to
+// which they are used: 4,000 cells with rows of 300 synapses, ten substeps, 16
+// spikes a step 3.9 us, without heavy words 4.2; 120 spikes 5.7 and 4.5; 600
+// spikes 18 and 5.2; one substep, rows of 600, 60 spikes 3.8 and 3.8.
+constexpr double kHeavyLoad = 64.0;
 constexpr uint32_t kPullUnit = 1024;  // ELL entries per dense-pull work unit (32 per lane)
 constexpr uint32_t kStdpUnit = 128;   // ELL cells per plasticity work unit (4 per lane)
 constexpr int kPullBlock = 1024;             // threads per k_pull block (one per SM)
@@ -229,6 +234,7 @@ struct StepArgs {
   int32_t bf16;
   int32_t substeps;
   uint32_t sms;                   // the device's SMs
+  uint32_t hv_busy;               // too many spikes of heavy words a step: launch without them
 };
 
 // Launch wrappers (sgb_kernels.cu).  All return the launch status.

@@ -217,6 +217,21 @@ static int derived_tables(Sim& s, void** p, size_t bytes, bool* ok) {
   return SGB_OK;
 }
 
+// Whether the stimulus keeps the heavy words too busy for one warp per block
+// (args.hv_busy): the spikes a step that their input cells' sources cause at
+// their present rates, over a repeating window's whole period.
+static void plan_heavy_load(Sim& s) {
+  double load = 0;
+  for (size_t k = 0; k < s.heavy_src.size(); ++k) {
+    const SrcDev& d = s.srcs[k];
+    double p = d.kind == SGB_INPUT_POISSON ? ldexp((double)d.thresh, -32) : d.cyc;
+    if (d.win_end > d.win_start && d.win_period > 0)
+      p *= std::min(1.0, (double)(d.win_end - d.win_start) / (double)d.win_period);
+    load += s.heavy_src[k] * std::min(1.0, p * s.cfg.substeps);
+  }
+  s.args.hv_busy = load > kHeavyLoad ? 1u : 0u;
+}
+
 // The fused kernel's heavy words: 32-cell words with a row of at least
 // kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
 // block has room for the words' synapses onto its cells (half of its shared
@@ -227,8 +242,9 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
                         const std::vector<uint32_t>& syn, const std::vector<float>& wf,
                         const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
   StepArgs& a = s.args;
-  a.hv_words = a.hv_cap = a.hv_grid = 0;
+  a.hv_words = a.hv_cap = a.hv_grid = a.hv_busy = 0;
   s.n_heavy_cells = 0;
+  s.heavy_src.clear();
   if (!fused) return SGB_OK;
   const uint32_t B = (uint32_t)s.persistent_blocks;
   std::vector<std::pair<uint64_t, uint32_t>> cand;  // {synapses, word}
@@ -301,6 +317,14 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   a.hv_off = (const uint16_t*)(hb + o_off);
   a.hv_syn = (const uint2*)(hb + o_syn);
   a.hv_grid = B;
+  s.heavy_src.assign(s.srcs.size(), 0.0);
+  for (size_t k = 0; k < s.srcs.size(); ++k) {
+    const InputSource& src = s.nets[s.src_net[k]].inputs[s.src_idx[k]];
+    const uint32_t base = s.segs[s.net_seg0[s.src_net[k]] + src.pop].base;
+    for (uint32_t id : src.ids)
+      if (index[(base + id) >> 5] != 0xFFFFu) s.heavy_src[k] += 1.0;
+  }
+  plan_heavy_load(s);
   return SGB_OK;
 }
 
@@ -1164,6 +1188,7 @@ int sim_set_rates(Sim& s, int32_t net, int32_t n, const float* rates) {
     p.rate_hz = rates[s.src_idx[k]];
     fill_source(s.srcs[k], p, s.cfg.dt_ms);
   }
+  plan_heavy_load(s);
   if (!s.srcs.empty()) {
     // The pinned staging copy is reused only after the chunks that may read it.
     const bool shared = s.stream != s.own_stream;
@@ -1815,6 +1840,7 @@ int sim_checkpoint(Sim& s, void* buf, int64_t size, bool load) {
       memcpy(s.srcs.data(), p, nsrc);
       memcpy(s.h_srcs, s.srcs.data(), nsrc);
       s.srcs_dirty = false;
+      plan_heavy_load(s);
       SGB_CUDA(cudaMemcpy((void*)s.args.srcs, s.h_srcs, nsrc, cudaMemcpyHostToDevice));
     }
     if (int rc = wait_copies()) return rc;

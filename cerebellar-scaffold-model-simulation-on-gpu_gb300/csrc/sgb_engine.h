@@ -67,6 +67,7 @@ struct Sim {
   size_t hist_bytes = 0;      // spike history + its summary
   int persistent_blocks = 0;
   std::vector<uint32_t> upd_words;  // host copy of args.upd_words
+  std::vector<double> heavy_src;    // stimulus sources' cells in heavy words
   int64_t n_heavy_cells = 0;        // cells of the fused kernel's heavy words
   // Plasticity (STDP) of plastic projections.
   void* d_plast = nullptr;

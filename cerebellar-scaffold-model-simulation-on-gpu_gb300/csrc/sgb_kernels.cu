@@ -2155,6 +2155,86 @@ __host__ __device__ constexpr uint32_t fused_max_threads(uint32_t w) {
   return 32u * ((fused_max_words(w) + w - 1u) / w + 2u);
 }
 
+// The heavy words' spikes of one step, when they are many, into a block's delay
+// line (k_persistent_fused), by one warp: listed, then 32 cells at a time, their
+// synapses dealt over the lanes, where one cell after another costs about 110
+// cycles each.  got: the lane's words, 32 apart.  Returns the synapses added.
+// 4,000 heavy cells: at 150 Hz (60 spikes a step) 10.3 -> 2.7 us per step with 128
+// synapses each, 8.2 -> 3.8 with 600; at 4 Hz in ten substeps (16 a step) 5.4 ->
+// 3.9.  Out of line for one word per warp, where inlined it costs the common step
+// 4 % (92,550 cells 1.70 us without it, 1.73 out of line, 1.77 inlined).
+constexpr uint32_t kBoardFew = 5;     // lanes with spiking cells, up to which they are few
+constexpr uint32_t kBoardList = 256;  // cells listed at a time
+__device__ __forceinline__ uint32_t board_many(uint4 gotv, const uint16_t* s_hoff, const uint2* s_hsyn, int2* s_line,
+                                               uint16_t* s_list, uint32_t at, uint32_t n_line, uint32_t n_cell) {
+  const uint32_t lane = threadIdx.x & 31u;
+  static_assert(kHeavyWords == 128, "four words per lane");
+  uint32_t got[4] = {gotv.x, gotv.y, gotv.z, gotv.w}, walked = 0;
+#pragma unroll 1
+  while (true) {
+    uint32_t n_sp = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) n_sp += __popc(got[k]);
+    uint32_t to = n_sp;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(kFull, to, o);
+      if (lane >= (uint32_t)o) to += v;
+    }
+    const uint32_t all = min(__shfl_sync(kFull, to, 31), kBoardList);
+    if (!all) return walked;
+    to -= n_sp;
+#pragma unroll
+    for (uint32_t k = 0; k < kHeavyWords / 32u; ++k)
+#pragma unroll 1
+      while (got[k] && to < kBoardList) {
+        s_list[to++] = (uint16_t)((32u * k + lane) * 32u + __ffs(got[k]) - 1u);
+        got[k] &= got[k] - 1u;
+      }
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t i0 = 0; i0 < all; i0 += 32u) {
+      uint32_t q0 = 0, len = 0;
+      if (i0 + lane < all) {
+        const uint32_t c = s_list[i0 + lane];
+        q0 = s_hoff[c];
+        len = s_hoff[c + 1u] - q0;
+      }
+      uint32_t incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+      }
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      const uint32_t base = q0 - (incl - len);  // of the owner's synapses, less its first piece
+#pragma unroll 1
+      for (uint32_t t0 = 0; t0 < total; t0 += 32u) {
+        const uint32_t t = min(t0 + lane, total - 1u);
+        uint32_t owner = 0;
+#pragma unroll
+        for (uint32_t d = 16; d; d >>= 1)
+          if (__shfl_sync(kFull, incl, owner + d - 1u) <= t) owner += d;
+        const uint32_t q = __shfl_sync(kFull, base, owner) + t;
+        if (t0 + lane < total) {
+          const uint2 e = s_hsyn[q];  // {cell | delay << 10 | accumulator << 14, increment}
+          uint32_t slot = at + ((e.x >> 10) & 15u);
+          if (slot >= n_line) slot -= n_line;
+          atomicAdd(reinterpret_cast<int*>(s_line + slot * n_cell + (e.x & 1023u)) + (e.x >> 14), (int)e.y);
+        }
+      }
+      walked += total;
+    }
+    __syncwarp();
+  }
+}
+
+__device__ __noinline__ uint32_t board_many_call(uint4 gotv, const uint16_t* s_hoff, const uint2* s_hsyn,
+                                                 int2* s_line, uint16_t* s_list, uint32_t at, uint32_t n_line,
+                                                 uint32_t n_cell) {
+  return board_many(gotv, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell);
+}
+
 // TL: the step's timeline -- 0 spikes in their own step; for one-substep steps
 // 1 late push, 2 late push with a split grid barrier (see the loops below).
 // W: words per warp.  A warp that holds two words shares a step's bookkeeping
@@ -2182,6 +2262,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
   // periodic sources that fire.
   __shared__ uint2 s_on[2][kOnSubsteps];
   __shared__ int s_ok[2], s_board_ok;
+  __shared__ uint16_t s_list[kBoardList];  // board_many
   extern __shared__ uint2 s_dyn[];
   const uint32_t n_thr = blockDim.x, n_wrp = n_thr >> 5, last = n_wrp - 1u;  // fused_threads
   const uint32_t aide = last - 1u, nw = aide;  // nw: warps that may hold words
@@ -2543,6 +2624,16 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
         }
         __nanosleep(32);
       }
+    }
+    uint32_t nz = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) nz |= got[k];
+    const uint32_t busy = __popc(__ballot_sync(kFull, nz != 0u));
+    if (busy > kBoardFew) {
+      const uint4 g = make_uint4(got[0], got[1], got[2], got[3]);
+      walked += W == 1u ? board_many_call(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell)
+                        : board_many(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell);
+      return;
     }
 #pragma unroll
     for (uint32_t k = 0; k < kHeavyWords / 32u; ++k) {
@@ -3016,6 +3107,9 @@ cudaError_t launch_persistent(const StepArgs& a, uint32_t n_steps, int blocks, c
   uint32_t n = n_steps;
   void* params[] = {&args, &n};
   const int kind = persistent_kernel_kind(a, blocks);
+  // Without heavy words every row is pushed by its cell's block; the delay line
+  // is handed back to the ring at a launch's end, so launches may differ.
+  if (a.hv_busy) args.hv_words = 0;
   if (kind == SGB_KERNEL_RESIDENT && a.pull_smem)
     return cudaLaunchCooperativeKernel(pull_kernel(a, blocks), dim3(blocks),
                                        dim3(pull_threads(a, blocks)), params, a.pull_smem, s);

@@ -46,3 +46,44 @@ def check(net, chunks, kernel, substeps=1, bf16=False):
 @pytest.mark.parametrize("substeps", [1, 10])
 def test_general(rate, one_word, substeps):
     check(net_of(150_000, [0, 1, 2, 5], 20_000, rate, 4, one_word), [1, 20], 1, substeps)
+
+
+def burst_net(n_src, fan, n_lif, d_max, quiet=2.0, seed=4):
+    """Source cells with `fan` synapses each that all fire in one step of a hundred."""
+    net = net_of(n_src, [fan], n_lif, 40.0, d_max, seed=seed)
+    net.set_input_stim(0, None, rate_hz=1e4, win_period_ms=10.0, win_start_ms=1.0, win_end_ms=1.1)
+    net.set_input_stim(0, None, kind=sg.INPUT_PERIODIC, rate_hz=quiet)
+    return net
+
+
+@pytest.mark.parametrize("n_src,fan,n_lif", [(4096, 130, 3000), (600, 700, 4800), (300, 256, 120_000)])
+@pytest.mark.parametrize("substeps,timeline", [(1, 0), (1, 1), (1, 2), (2, None)])
+def test_heavy_bursts(n_src, fan, n_lif, substeps, timeline, tmp_path):
+    """From no heavy spike in a step to all of them at once."""
+    from test_gpu_fused_blocks import check as check_fused
+
+    assert check_fused(burst_net(n_src, fan if substeps == 1 else max(fan, 256), n_lif, 5), 3, [1, 3, 8, 30, 70],
+                       substeps=substeps, timeline=timeline, tmp_path=tmp_path) > 0
+
+
+@pytest.mark.parametrize("substeps", [1, 10])
+def test_rates_across_the_heavy_limit(substeps):
+    """Launches with heavy words and without, in turn, as the rates change."""
+    net = net_of(3000, [300], 6000, 20.0, 5)
+    sim = sg.Simulation([net], [5], exec_mode=sg.EXEC_PERSISTENT, substeps=substeps, chunk_steps=16,
+                        default_prop=sg.PROP_CSR)
+    assert sim.info().step_kernel == 3 and sim.info().shard_cells > 0
+    o = oracle_py.Oracle(oracle_py.describe(net), seed=5, substeps=substeps)
+    for rate in (20.0, 900.0, 5.0, 2000.0, 0.0, 300.0, 12.0):
+        sim.set_input_freq(0, [rate])
+        o.set_rates([rate])
+        assert np.array_equal(sim.loop_n_steps(11)[0], o.run(11, 1 << 22)[0])
+        ck = sim.save_checkpoint()
+        sim.run(3)
+        sim.load_checkpoint(ck)
+    u, g, _ = sim.state()
+    eu, eg, _ = o.state()
+    assert np.array_equal(u.view(np.uint32), eu.view(np.uint32))
+    assert np.array_equal(g.view(np.uint32), eg.view(np.uint32))
+    assert sim.info().events == o.events()
+    sim.close()
