@@ -54,6 +54,16 @@ constexpr uint32_t kHeavyWords = 128;
 // spikes a step 3.9 us, without heavy words 4.2; 120 spikes 5.7 and 4.5; 600
 // spikes 18 and 5.2; one substep, rows of 600, 60 spikes 3.8 and 3.8.
 constexpr double kHeavyLoad = 64.0;
+// Longest row that its cell's warp pushes by itself, and shorter where rows
+// between the two are expected to cause more than kDirectLoad spikes a substep
+// (LIF cells at kDirectLifHz): one warp's rows follow one another, a block's items
+// run side by side behind a barrier.  20,000 cells with 140 synapses, 6 such
+// spikes a step, 2.22 us by themselves and 1.94 as items, 48 spikes 2.9 and 2.2,
+// 240 spikes 4.4 and 3.0; 4,000 with 120 synapses, 12 spikes 2.2 and 2.0; but
+// scaffolds with 1.5 spikes a step (139k cells) 2.0 and 2.2, with 10 in ten
+// substeps (97k cells) 4.3 and 4.5.
+constexpr uint32_t kDirectRow = 256, kDirectRowBusy = 64;
+constexpr double kDirectLoad = 4.0, kDirectLifHz = 10.0;
 constexpr uint32_t kPullUnit = 1024;  // ELL entries per dense-pull work unit (32 per lane)
 constexpr uint32_t kStdpUnit = 128;   // ELL cells per plasticity work unit (4 per lane)
 constexpr int kPullBlock = 1024;             // threads per k_pull block (one per SM)
@@ -234,6 +244,7 @@ struct StepArgs {
   int32_t bf16;
   int32_t substeps;
   uint32_t sms;                   // the device's SMs
+  uint32_t direct_row;            // fused kernel: longest row that its cell's warp pushes by itself
   uint32_t hv_busy;               // too many spikes of heavy words a step: launch without them
 };
 

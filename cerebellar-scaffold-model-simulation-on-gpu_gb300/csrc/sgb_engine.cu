@@ -217,19 +217,54 @@ static int derived_tables(Sim& s, void** p, size_t bytes, bool* ok) {
   return SGB_OK;
 }
 
-// Whether the stimulus keeps the heavy words too busy for one warp per block
-// (args.hv_busy): the spikes a step that their input cells' sources cause at
-// their present rates, over a repeating window's whole period.
-static void plan_heavy_load(Sim& s) {
-  double load = 0;
+// What the stimulus at its present rates, over a repeating window's whole period,
+// means for the fused kernel's launches: whether the heavy words are too busy for
+// one warp per block (args.hv_busy), and the longest row that a cell's warp pushes
+// by itself (args.direct_row).
+static void plan_load(Sim& s) {
+  double heavy = 0, rows[2] = {s.row_lif[0] * kDirectLifHz * 1e-3 * s.cfg.dt_ms,
+                               s.row_lif[1] * kDirectLifHz * 1e-3 * s.cfg.dt_ms};
   for (size_t k = 0; k < s.heavy_src.size(); ++k) {
     const SrcDev& d = s.srcs[k];
     double p = d.kind == SGB_INPUT_POISSON ? ldexp((double)d.thresh, -32) : d.cyc;
     if (d.win_end > d.win_start && d.win_period > 0)
       p *= std::min(1.0, (double)(d.win_end - d.win_start) / (double)d.win_period);
-    load += s.heavy_src[k] * std::min(1.0, p * s.cfg.substeps);
+    heavy += s.heavy_src[k] * std::min(1.0, p * s.cfg.substeps);
+    for (int j = 0; j < 2; ++j) rows[j] += s.row_src[j][k] * std::min(1.0, p);
   }
-  s.args.hv_busy = load > kHeavyLoad ? 1u : 0u;
+  s.args.hv_busy = heavy > kHeavyLoad ? 1u : 0u;
+  s.args.direct_row = rows[s.args.hv_busy] > kDirectLoad ? kDirectRowBusy : kDirectRow;
+}
+
+// Counts the cells that plan_load weighs: row, the push table's row starts;
+// own_end, the ends of what a cell's block pushes (a heavy word's: its start).
+static void count_load(Sim& s, const std::vector<uint32_t>& row, const std::vector<uint32_t>& own_end) {
+  auto middle = [&](uint32_t c, uint32_t end) {
+    return end - row[c] > kDirectRowBusy && end - row[c] <= kDirectRow ? 1.0 : 0.0;
+  };
+  s.heavy_src.assign(s.srcs.size(), 0.0);
+  for (int j = 0; j < 2; ++j) {
+    s.row_src[j].assign(s.srcs.size(), 0.0);
+    s.row_lif[j] = 0;
+  }
+  for (const SegDev& d : s.segs) {
+    if (d.kind != kSegLif) continue;
+    for (uint32_t c = d.base; c < d.base + d.count; ++c) {
+      s.row_lif[0] += middle(c, own_end[c]);
+      s.row_lif[1] += middle(c, row[c + 1]);
+    }
+  }
+  for (size_t k = 0; k < s.srcs.size(); ++k) {
+    const InputSource& src = s.nets[s.src_net[k]].inputs[s.src_idx[k]];
+    const uint32_t base = s.segs[s.net_seg0[s.src_net[k]] + src.pop].base;
+    for (uint32_t id : src.ids) {
+      const uint32_t c = base + id;
+      if (own_end[c] < row[c + 1]) s.heavy_src[k] += 1.0;
+      s.row_src[0][k] += middle(c, own_end[c]);
+      s.row_src[1][k] += middle(c, row[c + 1]);
+    }
+  }
+  plan_load(s);
 }
 
 // The fused kernel's heavy words: 32-cell words with a row of at least
@@ -242,9 +277,8 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
                         const std::vector<uint32_t>& syn, const std::vector<float>& wf,
                         const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
   StepArgs& a = s.args;
-  a.hv_words = a.hv_cap = a.hv_grid = a.hv_busy = 0;
+  a.hv_words = a.hv_cap = a.hv_grid = 0;
   s.n_heavy_cells = 0;
-  s.heavy_src.clear();
   if (!fused) return SGB_OK;
   const uint32_t B = (uint32_t)s.persistent_blocks;
   std::vector<std::pair<uint64_t, uint32_t>> cand;  // {synapses, word}
@@ -317,14 +351,6 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   a.hv_off = (const uint16_t*)(hb + o_off);
   a.hv_syn = (const uint2*)(hb + o_syn);
   a.hv_grid = B;
-  s.heavy_src.assign(s.srcs.size(), 0.0);
-  for (size_t k = 0; k < s.srcs.size(); ++k) {
-    const InputSource& src = s.nets[s.src_net[k]].inputs[s.src_idx[k]];
-    const uint32_t base = s.segs[s.net_seg0[s.src_net[k]] + src.pop].base;
-    for (uint32_t id : src.ids)
-      if (index[(base + id) >> 5] != 0xFFFFu) s.heavy_src[k] += 1.0;
-  }
-  plan_heavy_load(s);
   return SGB_OK;
 }
 
@@ -413,6 +439,7 @@ static int upload_modes(Sim& s) {
   a.row_smem = 0;
   std::vector<uint32_t> own_end(row.begin() + 1, row.end());
   if (int rc = upload_heavy(s, fused, row, syn, wf, wh, own_end)) return rc;
+  count_load(s, row, own_end);
   // The ends go with the rows also without heavy words (captured steps).
   if (s.d_heavy)
     SGB_CUDA(cudaMemcpy(s.d_heavy, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
@@ -1188,7 +1215,7 @@ int sim_set_rates(Sim& s, int32_t net, int32_t n, const float* rates) {
     p.rate_hz = rates[s.src_idx[k]];
     fill_source(s.srcs[k], p, s.cfg.dt_ms);
   }
-  plan_heavy_load(s);
+  plan_load(s);
   if (!s.srcs.empty()) {
     // The pinned staging copy is reused only after the chunks that may read it.
     const bool shared = s.stream != s.own_stream;
@@ -1840,7 +1867,7 @@ int sim_checkpoint(Sim& s, void* buf, int64_t size, bool load) {
       memcpy(s.srcs.data(), p, nsrc);
       memcpy(s.h_srcs, s.srcs.data(), nsrc);
       s.srcs_dirty = false;
-      plan_heavy_load(s);
+      plan_load(s);
       SGB_CUDA(cudaMemcpy((void*)s.args.srcs, s.h_srcs, nsrc, cudaMemcpyHostToDevice));
     }
     if (int rc = wait_copies()) return rc;

@@ -67,7 +67,10 @@ struct Sim {
   size_t hist_bytes = 0;      // spike history + its summary
   int persistent_blocks = 0;
   std::vector<uint32_t> upd_words;  // host copy of args.upd_words
-  std::vector<double> heavy_src;    // stimulus sources' cells in heavy words
+  // Stimulus sources' cells in heavy words; with rows between kDirectRowBusy and
+  // kDirectRow (not in heavy words, in any); LIF cells with such rows, likewise.
+  std::vector<double> heavy_src, row_src[2];
+  double row_lif[2] = {0, 0};
   int64_t n_heavy_cells = 0;        // cells of the fused kernel's heavy words
   // Plasticity (STDP) of plastic projections.
   void* d_plast = nullptr;

@@ -2100,7 +2100,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 // the ring, so a launch leaves what the other kernels expect.
 //   Other rows are pushed by the spiking cell's own warp, from a copy of the
 // block's rows in shared memory (row_smem; rows past the capacity stay in
-// global memory); only rows over kDirectRow synapses, in a block that has any,
+// global memory); only rows over a.direct_row synapses, in a block that has any,
 // are cut into items for all of the block's warps, at the price of a block
 // barrier a step.
 //   A step's stimulus decisions share what does not depend on the cell: which
@@ -2110,7 +2110,6 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 // 16-bit weights 2.46 -> 1.73; 9,256 cells 1.70 -> 1.48; 152,700 cells (two words
 // a warp) 2.71 -> 2.08; 92,550 cells in steps of ten substeps 6.6 -> 4.4.
 constexpr uint32_t kBlockItems = 1024;  // push items per block and step (8 KiB)
-constexpr uint32_t kDirectRow = 256;    // longest row that its cell's warp pushes by itself
 constexpr uint32_t kSrcCache = 16;      // stimulus sources kept in shared memory
 constexpr uint32_t kOnSubsteps = 32;    // substeps whose source states are shared
 // Items are ranges of 2^a.item_log2 synapses (64 or 128) of a long row: (first
@@ -2433,7 +2432,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
   uint32_t used = 0;
   bool has_long = false;
 #pragma unroll
-  for (uint32_t k = 0; k < W; ++k) has_long |= row[k].y > kDirectRow;
+  for (uint32_t k = 0; k < W; ++k) has_long |= row[k].y > a.direct_row;
 #pragma unroll 1
   for (uint32_t pass = 0; pass < 2u && cap; ++pass) {
 #pragma unroll
@@ -2526,7 +2525,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
       if (mine) atomicAdd(&ctl->events, (unsigned long long)s_od[pick(k, cell[0], cell[W - 1])]);
       const uint32_t rx = pick(k, row[0].x, row[W - 1].x), ry = pick(k, row[0].y, row[W - 1].y);
       const uint32_t n = ry & 0x7FFFFFFFu;
-      uint32_t todo = __ballot_sync(kFull, mine && n != 0u && n <= kDirectRow);
+      uint32_t todo = __ballot_sync(kFull, mine && n != 0u && n <= a.direct_row);
 #pragma unroll 1
       while (todo) {
         const int src = __ffs(todo) - 1;
@@ -2537,7 +2536,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
       if (blk_long) {
         // Long rows: items of the block's list, and from here what it has no room for.
         uint32_t from = 0;
-        const bool is_long = mine && n > kDirectRow;
+        const bool is_long = mine && n > a.direct_row;
         if (is_long) {
           const uint32_t nit = (n + chunk - 1u) >> clog;
           const uint32_t off = atomicAdd(&s_n[rel & 1u], nit);

@@ -87,3 +87,25 @@ def test_rates_across_the_heavy_limit(substeps):
     assert np.array_equal(g.view(np.uint32), eg.view(np.uint32))
     assert sim.info().events == o.events()
     sim.close()
+
+
+@pytest.mark.parametrize("substeps,fans", [(1, [0, 1, 63, 64, 65, 100, 127]), (1, [64, 65, 128, 129, 256, 257, 300]),
+                                           (10, [5, 64, 65, 200, 255])])
+@pytest.mark.parametrize("n_lif", [7000, 120_000])
+def test_rates_across_the_direct_limit(substeps, fans, n_lif):
+    """Rows of middle length pushed by their cells' warps and as items, in turn, as the rates change."""
+    net = net_of(5000, fans, n_lif, 20.0, 5)
+    sim = sg.Simulation([net], [5], exec_mode=sg.EXEC_PERSISTENT, substeps=substeps, chunk_steps=16,
+                        default_prop=sg.PROP_CSR)
+    assert sim.info().step_kernel == 3
+    o = oracle_py.Oracle(oracle_py.describe(net), seed=5, substeps=substeps)
+    for rate in (20.0, 900.0, 1.0, 150.0, 0.0, 40.0):
+        sim.set_input_freq(0, [rate])
+        o.set_rates([rate])
+        assert np.array_equal(sim.loop_n_steps(11)[0], o.run(11, 1 << 22)[0])
+    u, g, _ = sim.state()
+    eu, eg, _ = o.state()
+    assert np.array_equal(u.view(np.uint32), eu.view(np.uint32))
+    assert np.array_equal(g.view(np.uint32), eg.view(np.uint32))
+    assert sim.info().events == o.events()
+    sim.close()
