@@ -49,6 +49,11 @@ constexpr uint32_t kPushChunk = 256;  // synapses per push work item (8 per lane
 constexpr uint32_t kHeavyMin = 128;
 constexpr uint32_t kHeavyMinSub = 256;
 constexpr uint32_t kHeavyWords = 128;
+// Shared memory that heavy words leave to the other push rows, which may as well
+// stay in global memory.  4,000 cells with rows of 600 synapses: 2.02 us per step
+// with heavy words in half of the shared memory, 1.60 so; 2,000 with rows of
+// 2,500, 3.74 and 3.01; 138,825 scaffold cells 2.01 and 1.97.
+constexpr size_t kRowRest = 8192;
 // Spikes a step that the stimulus is expected to cause in heavy words, up to
 // which they are used: 4,000 cells with rows of 300 synapses, ten substeps, 16
 // spikes a step 3.9 us, without heavy words 4.2; 120 spikes 5.7 and 4.5; 600

@@ -269,8 +269,8 @@ static void count_load(Sim& s, const std::vector<uint32_t>& row, const std::vect
 
 // The fused kernel's heavy words: 32-cell words with a row of at least
 // kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
-// block has room for the words' synapses onto its cells (half of its shared
-// memory with the delay line; the push rows get the rest).  Fills the handle's
+// block has room for the words' synapses onto its cells (all of its shared memory
+// but kRowRest, with the delay line; the push rows get the rest).  Fills the handle's
 // tables and takes the words' rows out of own_end (the end of what a cell's
 // block pushes; the caller uploads it to the tables' start).
 static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
@@ -293,7 +293,7 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   std::vector<uint32_t> slot_of_word(s.n_words, 0);
   for (size_t ws = 0; ws < s.upd_words.size(); ++ws) slot_of_word[s.upd_words[ws]] = (uint32_t)ws;
   auto target = [&](uint32_t q) { return slot_of_word[(syn[q] & kPushPostMask) >> 5]; };
-  const size_t budget = fused_row_smem_max() / 2;
+  const size_t budget = fused_row_smem_max() - kRowRest;
   std::vector<uint32_t> count(B, 0), add(B), words;
   for (const auto& cw : cand) {
     if (words.size() == kHeavyWords) break;
