@@ -54,6 +54,12 @@ constexpr uint32_t kHeavyWords = 128;
 // with heavy words in half of the shared memory, 1.60 so; 2,000 with rows of
 // 2,500, 3.74 and 3.01; 138,825 scaffold cells 2.01 and 1.97.
 constexpr size_t kRowRest = 8192;
+// A word with a row of at least kHeavyFar synapses is heavy also when its synapses
+// no longer fit: those are read from global memory (the kernel's FAR form, for
+// these handles only: one that looks where each synapse lies costs scaffolds 1 to
+// 4 %).  2,000 cells with rows of 2,500 synapses, half of them held: 3.0 us per
+// step with the rest pushed by their own blocks, 1.8 so; at 30 Hz 5.6 and 2.8.
+constexpr uint32_t kHeavyFar = 1024;
 // Spikes a step that the stimulus is expected to cause in heavy words, up to
 // which they are used: 4,000 cells with rows of 300 synapses, ten substeps, 16
 // spikes a step 3.9 us, without heavy words 4.2; 120 spikes 5.7 and 4.5; 600
@@ -241,6 +247,7 @@ struct StepArgs {
   uint32_t row_smem;              // fused persistent kernel: shared-memory bytes for push rows (0: none)
   // Heavy words of the fused persistent kernel, for a grid of hv_grid blocks.
   uint32_t hv_words, hv_grid, hv_cap;  // words (0: none); most synapses of them onto one block
+  uint32_t hv_held;               // how many of those a block holds in shared memory
   const uint32_t* push_split;     // [n_pad] end of the part of a row its block pushes
   const uint16_t* hv_index;       // [n_words] index of a heavy word, 0xFFFF: not heavy
   const uint16_t* hv_off;         // [hv_grid][hv_words * 32 + 1] first synapse of each heavy cell

@@ -270,26 +270,31 @@ static void count_load(Sim& s, const std::vector<uint32_t>& row, const std::vect
 // The fused kernel's heavy words: 32-cell words with a row of at least
 // kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
 // block has room for the words' synapses onto its cells (all of its shared memory
-// but kRowRest, with the delay line; the push rows get the rest).  Fills the handle's
+// but kRowRest, with the delay line; the push rows get the rest) or a row reaches
+// kHeavyFar.  Fills the handle's
 // tables and takes the words' rows out of own_end (the end of what a cell's
 // block pushes; the caller uploads it to the tables' start).
 static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
                         const std::vector<uint32_t>& syn, const std::vector<float>& wf,
                         const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
   StepArgs& a = s.args;
-  a.hv_words = a.hv_cap = a.hv_grid = 0;
+  a.hv_words = a.hv_cap = a.hv_held = a.hv_grid = 0;
   s.n_heavy_cells = 0;
   if (!fused) return SGB_OK;
   const uint32_t B = (uint32_t)s.persistent_blocks;
-  std::vector<std::pair<uint64_t, uint32_t>> cand;  // {synapses, word}
+  struct Cand {
+    uint64_t synapses;
+    uint32_t word, longest;
+  };
+  std::vector<Cand> cand;
   const uint32_t least = a.substeps == 1 ? kHeavyMin : kHeavyMinSub;
   for (uint32_t w : s.upd_words) {
     uint32_t longest = 0;
     for (uint32_t c = w * 32; c < w * 32 + 32; ++c) longest = std::max(longest, row[c + 1] - row[c]);
-    if (longest >= least) cand.push_back({(uint64_t)(row[w * 32 + 32] - row[w * 32]), w});
+    if (longest >= least) cand.push_back({(uint64_t)(row[w * 32 + 32] - row[w * 32]), w, longest});
   }
   if (cand.empty()) return SGB_OK;
-  std::stable_sort(cand.begin(), cand.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::stable_sort(cand.begin(), cand.end(), [](const auto& x, const auto& y) { return x.synapses > y.synapses; });
   std::vector<uint32_t> slot_of_word(s.n_words, 0);
   for (size_t ws = 0; ws < s.upd_words.size(); ++ws) slot_of_word[s.upd_words[ws]] = (uint32_t)ws;
   auto target = [&](uint32_t q) { return slot_of_word[(syn[q] & kPushPostMask) >> 5]; };
@@ -298,18 +303,24 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   for (const auto& cw : cand) {
     if (words.size() == kHeavyWords) break;
     std::fill(add.begin(), add.end(), 0u);
-    for (uint32_t q = row[cw.second * 32]; q < row[cw.second * 32 + 32]; ++q) add[target(q) % B]++;
+    for (uint32_t q = row[cw.word * 32]; q < row[cw.word * 32 + 32]; ++q) add[target(q) % B]++;
     uint32_t most = 0;
     for (uint32_t b = 0; b < B; ++b) most = std::max(most, count[b] + add[b]);
+    if (most > 0xFFFFu) break;
     a.hv_words = (uint32_t)words.size() + 1;
-    a.hv_cap = most;
-    if (most > 0xFFFFu || fused_heavy_bytes(a, s.persistent_blocks) > budget) break;
+    a.hv_held = most;
+    if (fused_heavy_bytes(a, s.persistent_blocks) > budget) {
+      a.hv_held = 0;
+      if (cw.longest < kHeavyFar || fused_heavy_bytes(a, s.persistent_blocks) > budget) break;
+    }
     for (uint32_t b = 0; b < B; ++b) count[b] += add[b];
-    words.push_back(cw.second);
+    words.push_back(cw.word);
   }
   a.hv_words = (uint32_t)words.size();
   a.hv_cap = *std::max_element(count.begin(), count.end());
+  a.hv_held = 0;
   if (words.empty()) return SGB_OK;
+  a.hv_held = std::min<uint32_t>(a.hv_cap, (uint32_t)((budget - fused_heavy_bytes(a, s.persistent_blocks)) / sizeof(uint2)));
   const uint32_t n_off = a.hv_words * 32 + 1;
   std::vector<uint16_t> index(s.n_words, 0xFFFF), off((size_t)B * n_off, 0);
   std::vector<uint2> list((size_t)B * a.hv_cap, make_uint2(0, 0));
@@ -333,11 +344,17 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   }
   const size_t o_idx = align_up((size_t)s.n_pad * 4, 256), o_off = align_up(o_idx + index.size() * 2, 256);
   const size_t o_syn = align_up(o_off + (size_t)B * (kHeavyWords * 32u + 1u) * 2, 256);
-  const size_t most_cap = std::min<size_t>(budget / sizeof(uint2), (size_t)std::max<int64_t>(s.n_syn, 1));
+  // The most that any modes can put into a block's list: every synapse onto its cells.
+  std::vector<size_t> onto(B, 0);
+  for (const ProjTables& t : s.ptab) {
+    const uint32_t post_base = s.segs[t.post_seg].base;
+    for (uint32_t id : s.nets[t.net].projs[t.proj].post_idx) onto[slot_of_word[(post_base + id) >> 5] % B]++;
+  }
+  const size_t most_cap = std::min<size_t>(0xFFFFu, *std::max_element(onto.begin(), onto.end()));
   bool ok;
   if (int rc = derived_tables(s, &s.d_heavy, o_syn + B * most_cap * sizeof(uint2), &ok)) return rc;
   if (!ok) {  // every row stays with its cell's block
-    a.hv_words = a.hv_cap = 0;
+    a.hv_words = a.hv_cap = a.hv_held = 0;
     s.n_heavy_cells = 0;
     own_end.assign(row.begin() + 1, row.end());
     return SGB_OK;

@@ -2135,14 +2135,14 @@ __device__ __forceinline__ void source_states(const SrcDev* srcs, uint2* on, uin
 }
 
 // Shared memory of the heavy words: the line, where each heavy cell's synapses
-// start, and up to hv_cap of them.
+// start, and up to hv_held of them.
 __host__ __device__ __forceinline__ uint32_t hv_line_slots(const StepArgs& a) { return a.max_delay + 1u; }
 __host__ __device__ __forceinline__ size_t hv_bytes(const StepArgs& a, uint32_t blocks) {
   if (!a.hv_words) return 0;
   const size_t cells = ((size_t)a.n_upd_words + blocks - 1u) / blocks * 32u;
   const size_t line = hv_line_slots(a) * cells * sizeof(int2);
   const size_t off = ((size_t)(a.hv_words * 32u + 1u) * sizeof(uint16_t) + 15) & ~(size_t)15;
-  return line + off + (size_t)a.hv_cap * sizeof(uint2);
+  return line + off + (size_t)a.hv_held * sizeof(uint2);
 }
 
 // Words of a block, at most: one per warp up to kFusedSingle, else two.
@@ -2164,8 +2164,10 @@ __host__ __device__ constexpr uint32_t fused_max_threads(uint32_t w) {
 // 4 % (92,550 cells 1.70 us without it, 1.73 out of line, 1.77 inlined).
 constexpr uint32_t kBoardFew = 5;     // lanes with spiking cells, up to which they are few
 constexpr uint32_t kBoardList = 256;  // cells listed at a time
+template <bool FAR>
 __device__ __forceinline__ uint32_t board_many(uint4 gotv, const uint16_t* s_hoff, const uint2* s_hsyn, int2* s_line,
-                                               uint16_t* s_list, uint32_t at, uint32_t n_line, uint32_t n_cell) {
+                                               uint16_t* s_list, uint32_t at, uint32_t n_line, uint32_t n_cell,
+                                               const uint2* far, uint32_t held) {
   const uint32_t lane = threadIdx.x & 31u;
   static_assert(kHeavyWords == 128, "four words per lane");
   uint32_t got[4] = {gotv.x, gotv.y, gotv.z, gotv.w}, walked = 0;
@@ -2216,7 +2218,8 @@ __device__ __forceinline__ uint32_t board_many(uint4 gotv, const uint16_t* s_hof
           if (__shfl_sync(kFull, incl, owner + d - 1u) <= t) owner += d;
         const uint32_t q = __shfl_sync(kFull, base, owner) + t;
         if (t0 + lane < total) {
-          const uint2 e = s_hsyn[q];  // {cell | delay << 10 | accumulator << 14, increment}
+          // {cell | delay << 10 | accumulator << 14, increment}
+          const uint2 e = FAR && q >= held ? __ldg(far + q) : s_hsyn[q];
           uint32_t slot = at + ((e.x >> 10) & 15u);
           if (slot >= n_line) slot -= n_line;
           atomicAdd(reinterpret_cast<int*>(s_line + slot * n_cell + (e.x & 1023u)) + (e.x >> 14), (int)e.y);
@@ -2228,10 +2231,11 @@ __device__ __forceinline__ uint32_t board_many(uint4 gotv, const uint16_t* s_hof
   }
 }
 
+template <bool FAR>
 __device__ __noinline__ uint32_t board_many_call(uint4 gotv, const uint16_t* s_hoff, const uint2* s_hsyn,
                                                  int2* s_line, uint16_t* s_list, uint32_t at, uint32_t n_line,
-                                                 uint32_t n_cell) {
-  return board_many(gotv, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell);
+                                                 uint32_t n_cell, const uint2* far, uint32_t held) {
+  return board_many<FAR>(gotv, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell, far, held);
 }
 
 // TL: the step's timeline -- 0 spikes in their own step; for one-substep steps
@@ -2242,7 +2246,8 @@ __device__ __noinline__ uint32_t board_many_call(uint4 gotv, const uint16_t* s_h
 // memory this kernel takes, little is left for L1, and a spilled register
 // costs an L2 round trip).  Two more warps hold no word: the last keeps the grid
 // barrier, the one before it reads the board and prepares the sources.
-template <bool BF16, uint32_t TL, uint32_t W>
+// FAR: some of the heavy words' synapses are in global memory.
+template <bool BF16, uint32_t TL, uint32_t W, bool FAR>
 __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(StepArgs a,
                                                                               uint32_t n_steps) {
   __shared__ uint2 s_items[kBlockItems];
@@ -2272,7 +2277,8 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
   int2* s_line = reinterpret_cast<int2*>(s_dyn);  // [n_line][n_cell]
   uint16_t* s_hoff = reinterpret_cast<uint16_t*>(s_line + (heavy ? n_line * n_cell : 0u));
   uint2* s_rows = s_dyn + hv_bytes(a, gridDim.x) / sizeof(uint2);
-  uint2* s_hsyn = s_rows - (heavy ? a.hv_cap : 0u);
+  uint2* s_hsyn = s_rows - (heavy ? a.hv_held : 0u);
+  const uint2* far = FAR ? a.hv_syn + (size_t)blockIdx.x * a.hv_cap : nullptr;
   const SegDev* segs = a.n_segs <= kSegCache ? s_seg : a.segs;
   const SrcDev* srcs = a.n_srcs <= kSrcCache ? s_src : a.srcs;
   const bool shared_src = a.n_srcs <= kSrcCache && a.substeps <= (int)kOnSubsteps;
@@ -2337,7 +2343,7 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
     const uint32_t n = min((uint32_t)__ldg(off + n_off - 1u), a.hv_cap);
     for (uint32_t j = threadIdx.x; j < n_off; j += n_thr) s_hoff[j] = (uint16_t)min((uint32_t)__ldg(off + j), n);
     const uint2* src = a.hv_syn + (size_t)blockIdx.x * a.hv_cap;
-    for (uint32_t j = threadIdx.x; j < n; j += n_thr) s_hsyn[j] = __ldg(src + j);
+    for (uint32_t j = threadIdx.x; j < (FAR ? min(n, a.hv_held) : n); j += n_thr) s_hsyn[j] = __ldg(src + j);
   }
   uint32_t stim = 0;  // bit k: the thread's cell of word k is a stimulated input cell
 #pragma unroll
@@ -2630,8 +2636,8 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
     const uint32_t busy = __popc(__ballot_sync(kFull, nz != 0u));
     if (busy > kBoardFew) {
       const uint4 g = make_uint4(got[0], got[1], got[2], got[3]);
-      walked += W == 1u ? board_many_call(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell)
-                        : board_many(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell);
+      walked += W == 1u ? board_many_call<FAR>(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell, far, a.hv_held)
+                        : board_many<FAR>(g, s_hoff, s_hsyn, s_line, s_list, at, n_line, n_cell, far, a.hv_held);
       return;
     }
 #pragma unroll
@@ -2651,7 +2657,8 @@ __global__ void __launch_bounds__(fused_max_threads(W), 1) k_persistent_fused(St
           walked += q1 - s_hoff[c];
 #pragma unroll 1
           for (uint32_t q = s_hoff[c] + lane; q < q1; q += 32u) {
-            const uint2 e = s_hsyn[q];  // {cell | delay << 10 | accumulator << 14, increment}
+            // {cell | delay << 10 | accumulator << 14, increment}
+            const uint2 e = FAR && q >= a.hv_held ? __ldg(far + q) : s_hsyn[q];
             uint32_t slot = at + ((e.x >> 10) & 15u);
             if (slot >= n_line) slot -= n_line;
             atomicAdd(reinterpret_cast<int*>(s_line + slot * n_cell + (e.x & 1023u)) + (e.x >> 14), (int)e.y);
@@ -2952,13 +2959,14 @@ static size_t dyn_smem_max(const void* fn) {
   return ((size_t)optin - fa.sharedSizeBytes) & ~(size_t)255;
 }
 
-// The fused kernel's forms: [BF16][timeline][words per warp - 1].
-#define SGB_FUSED_FORMS(B)                                                      \
-  (const void*)k_persistent_fused<B, 0, 1>, (const void*)k_persistent_fused<B, 0, 2>,     \
-      (const void*)k_persistent_fused<B, 1, 1>, (const void*)k_persistent_fused<B, 1, 2>, \
-      (const void*)k_persistent_fused<B, 2, 1>, (const void*)k_persistent_fused<B, 2, 2>
+// The fused kernel's forms: [FAR][BF16][timeline][words per warp - 1].
+#define SGB_FUSED_FORMS(B, F)                                                        \
+  (const void*)k_persistent_fused<B, 0, 1, F>, (const void*)k_persistent_fused<B, 0, 2, F>,     \
+      (const void*)k_persistent_fused<B, 1, 1, F>, (const void*)k_persistent_fused<B, 1, 2, F>, \
+      (const void*)k_persistent_fused<B, 2, 1, F>, (const void*)k_persistent_fused<B, 2, 2, F>
 constexpr uint32_t kFusedForms = 6;
-static const void* const kFusedKernels[] = {SGB_FUSED_FORMS(false), SGB_FUSED_FORMS(true)};
+static const void* const kFusedKernels[] = {SGB_FUSED_FORMS(false, false), SGB_FUSED_FORMS(true, false),
+                                            SGB_FUSED_FORMS(false, true), SGB_FUSED_FORMS(true, true)};
 #undef SGB_FUSED_FORMS
 
 cudaError_t pull_setup() {
@@ -3026,12 +3034,13 @@ uint32_t fused_item_log2(const StepArgs& a) {
 }
 
 static const void* fused_kernel(const StepArgs& a, int blocks) {
-  return kFusedKernels[(a.bf16 ? kFusedForms : 0u) + 2u * fused_timeline(a) + fused_per_warp(a, blocks) - 1u];
+  const uint32_t far = a.hv_words && a.hv_held < a.hv_cap ? 2u * kFusedForms : 0u;
+  return kFusedKernels[far + (a.bf16 ? kFusedForms : 0u) + 2u * fused_timeline(a) + fused_per_warp(a, blocks) - 1u];
 }
 
 static int fused_blocks_per_sm() {
   int n = 1 << 20;
-  for (uint32_t k = 0; k < 2u * kFusedForms; ++k) {
+  for (uint32_t k = 0; k < 4u * kFusedForms; ++k) {
     int f = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, kFusedKernels[k], (int)fused_max_threads(k % 2u + 1u), 0);
     n = f < n ? f : n;

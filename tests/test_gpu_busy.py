@@ -109,3 +109,16 @@ def test_rates_across_the_direct_limit(substeps, fans, n_lif):
     assert np.array_equal(g.view(np.uint32), eg.view(np.uint32))
     assert sim.info().events == o.events()
     sim.close()
+
+
+@pytest.mark.parametrize("n_lif,substeps,timeline,bf16", [
+    (60_000, 1, 0, False), (60_000, 1, 1, True), (60_000, 1, 2, False), (60_000, 10, None, False),
+    (120_000, 1, 0, True), (120_000, 1, 1, False), (120_000, 1, 2, True), (120_000, 3, None, False)])
+def test_rows_past_shared_memory(n_lif, substeps, timeline, bf16, tmp_path):
+    """Five million synapses of heavy words, about two thirds of which fit the blocks' shared memory."""
+    from test_gpu_fused_blocks import check as check_fused
+
+    net = net_of(2000, [2400, 2600], n_lif, 40.0, 4)
+    net.set_input_stim(0, np.arange(0, 2000, 3), rate_hz=1e4, win_period_ms=10.0, win_start_ms=2.0, win_end_ms=2.1)
+    heavy = check_fused(net, 3, [1, 3, 8, 30, 7], bf16=bf16, substeps=substeps, timeline=timeline, tmp_path=tmp_path)
+    assert heavy == 2000
