@@ -21,10 +21,9 @@
 //              double-buffered by step parity.  The fused persistent kernel
 //              keeps its items, and its blocks' push rows, in shared memory.
 //   push table one cell-major CSR over every projection in event-driven mode
-//              (all instances), each row's delay-1 synapses first, then its
-//              delay-2 synapses, then the rest: synapse
-//              word = padded post index | delay << 27 | accumulator << 31, plus
-//              the weight pre-multiplied by its accumulator's 2^S (exact
+//              (all instances), a row's synapses by projection: synapse word =
+//              padded post index | delay << 27 | accumulator << 31, plus the
+//              weight pre-multiplied by its accumulator's 2^S (exact
 //              power-of-two scaling) in FP32 or BF16.
 //   ELL tables per projection, post-major (dense pull): entry = (delay - 1) *
 //              n_pad + padded pre index, the offset of the pre cell's spike bit
@@ -41,13 +40,9 @@ constexpr int kPersistBlock = 1024;   // threads per block of the persistent ker
 constexpr uint32_t kPushChunk = 256;  // synapses per push work item (8 per lane)
 // Fused persistent kernel: 32-cell words that hold a row of at least kHeavyMin
 // synapses are delivered by the blocks of their targets (at most kHeavyWords).
-// One warp per block handles a step's heavy spikes one after another, so
-// exchange steps of several substeps, with as many times the spikes, leave
-// shorter rows to their own blocks (kHeavyMinSub; 97k cells, ten substeps,
-// rows of 147 synapses heavy 5.9 us per step, not heavy 4.6; one substep 1.71
-// and 1.91 us).
+// 97k scaffold cells, whose 2,500 mossy fibres have rows of 147: heavy 1.74 us per
+// step, not heavy 1.91; with ten substeps 4.21 and 4.30.
 constexpr uint32_t kHeavyMin = 128;
-constexpr uint32_t kHeavyMinSub = 256;
 constexpr uint32_t kHeavyWords = 128;
 // Shared memory that heavy words leave to the other push rows, which may as well
 // stay in global memory.  4,000 cells with rows of 600 synapses: 2.02 us per step

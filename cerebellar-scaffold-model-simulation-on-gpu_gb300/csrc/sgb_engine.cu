@@ -267,13 +267,12 @@ static void count_load(Sim& s, const std::vector<uint32_t>& row, const std::vect
   plan_load(s);
 }
 
-// The fused kernel's heavy words: 32-cell words with a row of at least
-// kHeavyMin (kHeavyMinSub) synapses, those with the most synapses first, as long as every
-// block has room for the words' synapses onto its cells (all of its shared memory
-// but kRowRest, with the delay line; the push rows get the rest) or a row reaches
-// kHeavyFar.  Fills the handle's
-// tables and takes the words' rows out of own_end (the end of what a cell's
-// block pushes; the caller uploads it to the tables' start).
+// The fused kernel's heavy words: 32-cell words with a row of at least kHeavyMin
+// synapses, those with the most synapses first, as long as every block has room
+// for the words' synapses onto its cells (all of its shared memory but kRowRest,
+// with the delay line; the push rows get the rest) or a row reaches kHeavyFar.
+// Fills the handle's tables and takes the words' rows out of own_end (the end of
+// what a cell's block pushes; the caller uploads it to the tables' start).
 static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
                         const std::vector<uint32_t>& syn, const std::vector<float>& wf,
                         const std::vector<uint16_t>& wh, std::vector<uint32_t>& own_end) {
@@ -287,11 +286,10 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
     uint32_t word, longest;
   };
   std::vector<Cand> cand;
-  const uint32_t least = a.substeps == 1 ? kHeavyMin : kHeavyMinSub;
   for (uint32_t w : s.upd_words) {
     uint32_t longest = 0;
     for (uint32_t c = w * 32; c < w * 32 + 32; ++c) longest = std::max(longest, row[c + 1] - row[c]);
-    if (longest >= least) cand.push_back({(uint64_t)(row[w * 32 + 32] - row[w * 32]), w, longest});
+    if (longest >= kHeavyMin) cand.push_back({(uint64_t)(row[w * 32 + 32] - row[w * 32]), w, longest});
   }
   if (cand.empty()) return SGB_OK;
   std::stable_sort(cand.begin(), cand.end(), [](const auto& x, const auto& y) { return x.synapses > y.synapses; });

@@ -2088,15 +2088,17 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 // scattered reductions leave one SM at about three cycles each).  So long rows
 // are not pushed by their block:
 //   Heavy words (32-cell words of long rows, chosen by the host).  Every block
-// keeps the heavy cells' synapses onto its own cells in shared memory, grouped
-// by heavy cell, and an own delay line of increments (s_line) for its cells.
+// keeps the heavy cells' synapses onto its own cells in shared memory (very long
+// rows' partly in global memory, FAR), grouped by heavy cell, and an own delay line of increments (s_line) for its cells.
 // A heavy word's spikes of step t go onto a board in global memory, one 64-bit
 // word {step tag, spike bits} per heavy word; in step t one warp of every
 // block reads the board, adds what its cells receive into its line's slots t +
 // d, d >= 1, and the block barrier that ends the step hands them to the update
 // of t + 1.  Bits and tag share a word, so the board needs no fence and no
 // barrier of its own.  A Golgi spike becomes ten additions in each block's
-// shared memory.  At the end of a launch the line's pending slots are added to
+// shared memory; many spikes at once are dealt over the warp's lanes (board_many).
+// When the stimulus alone keeps that warp too busy, a launch goes without heavy
+// words (a.hv_busy).  At the end of a launch the line's pending slots are added to
 // the ring, so a launch leaves what the other kernels expect.
 //   Other rows are pushed by the spiking cell's own warp, from a copy of the
 // block's rows in shared memory (row_smem; rows past the capacity stay in
@@ -2106,9 +2108,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 //   A step's stimulus decisions share what does not depend on the cell: which
 // sources are on or fire periodically in each substep is worked out once per
 // block, by that warp, a lane per source and substep (s_on).
-//   Per step, start of this design -> now: 92,550 cells 2.21 -> 1.69 us, with
-// 16-bit weights 2.46 -> 1.73; 9,256 cells 1.70 -> 1.48; 152,700 cells (two words
-// a warp) 2.71 -> 2.08; 92,550 cells in steps of ten substeps 6.6 -> 4.4.
+//   Per step, without heavy words and with every row as items -> now: 92,550 cells
+// 2.24 -> 1.74 us, with 16-bit weights 2.45 -> 1.75; 9,256 cells 1.71 -> 1.49;
+// 152,700 cells (two words a warp) 2.69 -> 2.03; 97,020 cells in steps of ten
+// substeps 6.84 -> 4.21.
 constexpr uint32_t kBlockItems = 1024;  // push items per block and step (8 KiB)
 constexpr uint32_t kSrcCache = 16;      // stimulus sources kept in shared memory
 constexpr uint32_t kOnSubsteps = 32;    // substeps whose source states are shared
