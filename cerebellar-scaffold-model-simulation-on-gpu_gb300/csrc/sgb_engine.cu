@@ -342,15 +342,18 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   }
   const size_t o_idx = align_up((size_t)s.n_pad * 4, 256), o_off = align_up(o_idx + index.size() * 2, 256);
   const size_t o_syn = align_up(o_off + (size_t)B * (kHeavyWords * 32u + 1u) * 2, 256);
-  // The most that any modes can put into a block's list: every synapse onto its cells.
-  std::vector<size_t> onto(B, 0);
-  for (const ProjTables& t : s.ptab) {
-    const uint32_t post_base = s.segs[t.post_seg].base;
-    for (uint32_t id : s.nets[t.net].projs[t.proj].post_idx) onto[slot_of_word[(post_base + id) >> 5] % B]++;
+  size_t bytes = 0;
+  if (!s.d_heavy) {
+    // The most that any modes can put into a block's list: every synapse onto its cells.
+    std::vector<size_t> onto(B, 0);
+    for (const ProjTables& t : s.ptab) {
+      const uint32_t post_base = s.segs[t.post_seg].base;
+      for (uint32_t id : s.nets[t.net].projs[t.proj].post_idx) onto[slot_of_word[(post_base + id) >> 5] % B]++;
+    }
+    bytes = o_syn + B * std::min<size_t>(0xFFFFu, *std::max_element(onto.begin(), onto.end())) * sizeof(uint2);
   }
-  const size_t most_cap = std::min<size_t>(0xFFFFu, *std::max_element(onto.begin(), onto.end()));
   bool ok;
-  if (int rc = derived_tables(s, &s.d_heavy, o_syn + B * most_cap * sizeof(uint2), &ok)) return rc;
+  if (int rc = derived_tables(s, &s.d_heavy, bytes, &ok)) return rc;
   if (!ok) {  // every row stays with its cell's block
     a.hv_words = a.hv_cap = a.hv_held = 0;
     s.n_heavy_cells = 0;
@@ -454,7 +457,7 @@ static int upload_modes(Sim& s) {
   a.row_smem = 0;
   std::vector<uint32_t> own_end(row.begin() + 1, row.end());
   if (int rc = upload_heavy(s, fused, row, syn, wf, wh, own_end)) return rc;
-  count_load(s, row, own_end);
+  if (fused) count_load(s, row, own_end);
   // The ends go with the rows also without heavy words (captured steps).
   if (s.d_heavy)
     SGB_CUDA(cudaMemcpy(s.d_heavy, own_end.data(), (size_t)s.n_pad * 4, cudaMemcpyHostToDevice));
