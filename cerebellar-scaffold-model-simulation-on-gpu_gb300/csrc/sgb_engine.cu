@@ -318,7 +318,8 @@ static int upload_heavy(Sim& s, bool fused, const std::vector<uint32_t>& row,
   a.hv_cap = *std::max_element(count.begin(), count.end());
   a.hv_held = 0;
   if (words.empty()) return SGB_OK;
-  a.hv_held = std::min<uint32_t>(a.hv_cap, (uint32_t)((budget - fused_heavy_bytes(a, s.persistent_blocks)) / sizeof(uint2)));
+  const size_t room = budget - fused_heavy_bytes(a, s.persistent_blocks);
+  a.hv_held = (uint32_t)std::min<size_t>(a.hv_cap, room / sizeof(uint2));
   const uint32_t n_off = a.hv_words * 32 + 1;
   std::vector<uint16_t> index(s.n_words, 0xFFFF), off((size_t)B * n_off, 0);
   std::vector<uint2> list((size_t)B * a.hv_cap, make_uint2(0, 0));

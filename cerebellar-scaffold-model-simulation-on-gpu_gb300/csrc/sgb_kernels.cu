@@ -2089,17 +2089,18 @@ __global__ void __launch_bounds__(MAXT, 1) k_persistent_pull(StepArgs a, uint32_
 // are not pushed by their block:
 //   Heavy words (32-cell words of long rows, chosen by the host).  Every block
 // keeps the heavy cells' synapses onto its own cells in shared memory (very long
-// rows' partly in global memory, FAR), grouped by heavy cell, and an own delay line of increments (s_line) for its cells.
-// A heavy word's spikes of step t go onto a board in global memory, one 64-bit
-// word {step tag, spike bits} per heavy word; in step t one warp of every
-// block reads the board, adds what its cells receive into its line's slots t +
-// d, d >= 1, and the block barrier that ends the step hands them to the update
-// of t + 1.  Bits and tag share a word, so the board needs no fence and no
-// barrier of its own.  A Golgi spike becomes ten additions in each block's
-// shared memory; many spikes at once are dealt over the warp's lanes (board_many).
-// When the stimulus alone keeps that warp too busy, a launch goes without heavy
-// words (a.hv_busy).  At the end of a launch the line's pending slots are added to
-// the ring, so a launch leaves what the other kernels expect.
+// rows' partly in global memory, FAR), grouped by heavy cell, and an own delay
+// line of increments (s_line) for its cells.  A heavy word's spikes of step t go
+// onto a board in global memory, one 64-bit word {step tag, spike bits} per heavy
+// word; in step t one warp of every block reads the board, adds what its cells
+// receive into its line's slots t + d, d >= 1, and the block barrier that ends
+// the step hands them to the update of t + 1.  Bits and tag share a word, so the
+// board needs no fence and no barrier of its own.  A Golgi spike becomes ten
+// additions in each block's shared memory; many spikes at once are dealt over the
+// warp's lanes (board_many).  When the stimulus alone keeps that warp too busy, a
+// launch goes without heavy words (a.hv_busy).  At the end of a launch the line's
+// pending slots are added to the ring, so a launch leaves what the other kernels
+// expect.
 //   Other rows are pushed by the spiking cell's own warp, from a copy of the
 // block's rows in shared memory (row_smem; rows past the capacity stay in
 // global memory); only rows over a.direct_row synapses, in a block that has any,
